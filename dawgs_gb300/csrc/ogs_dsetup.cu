@@ -74,8 +74,9 @@ inline unsigned rblocks(int64_t n) {
 }
 
 // key = |id| (0 for zero ids), val = local index.
+// code (may be null): INT32_MIN for zero ids (k_fill writes the others').
 __global__ void k_keys(const int64_t* __restrict__ ids, int64_t n, uint64_t* __restrict__ key,
-                       int32_t* __restrict__ val, Counters* c) {
+                       int32_t* __restrict__ val, int32_t* __restrict__ code, Counters* c) {
   using RU = cub::BlockReduce<unsigned long long, kT>;
   __shared__ typename RU::TempStorage tmp;
   unsigned long long m = 0, zeros = 0;
@@ -86,6 +87,7 @@ __global__ void k_keys(const int64_t* __restrict__ ids, int64_t n, uint64_t* __r
     bad |= (id == INT64_MIN);
     const uint64_t a = static_cast<uint64_t>(id < 0 ? -id : id);
     zeros += (id == 0);
+    if (code && id == 0) code[i] = INT32_MIN;
     m = a > m ? a : m;
     key[i] = a;
     val[i] = static_cast<int32_t>(i);
@@ -171,13 +173,15 @@ __global__ void k_rows(const int32_t* __restrict__ gfirst, const int32_t* __rest
   degN[r] = gpos[g];
 }
 
-// Each member to its slot: T map always, N map for positive members of a
+// Each member to its slot (and, with `code`, each node's row and N membership
+// for the node words): T map always, N map for positive members of a
 // Signed handle.  Members of a group are in ascending local index already.
 __global__ void k_fill(const int32_t* __restrict__ gincl, const int32_t* __restrict__ gstart,
                        const int32_t* __restrict__ grow, const int32_t* __restrict__ val,
                        const int32_t* __restrict__ pos, const int32_t* __restrict__ pos_ex,
                        const int32_t* __restrict__ rsT, const int32_t* __restrict__ rsN, int64_t nnz, int signed_maps,
-                       int32_t* __restrict__ ciT, int32_t* __restrict__ ciN) {
+                       int32_t* __restrict__ ciT, int32_t* __restrict__ ciN, int32_t* __restrict__ code,
+                       uint8_t* __restrict__ nmem) {
   const int64_t i = static_cast<int64_t>(blockIdx.x) * kT + threadIdx.x;
   if (i >= nnz) return;
   const int32_t g = gincl[i] - 1;
@@ -185,6 +189,10 @@ __global__ void k_fill(const int32_t* __restrict__ gincl, const int32_t* __restr
   const int32_t r = grow[g];
   ciT[rsT[r] + (static_cast<int32_t>(i) - s)] = val[i];
   if (signed_maps && pos[i]) ciN[rsN[r] + (pos_ex[i] - pos_ex[s])] = val[i];
+  if (code) {
+    code[val[i]] = i == s ? r : ~r;
+    nmem[val[i]] = static_cast<uint8_t>(pos[i]);
+  }
 }
 
 // unique: the first member of each group keeps +|id|, the rest get -|id|.
@@ -341,6 +349,36 @@ __global__ void k_wemask(const Tile* __restrict__ wt, int64_t nw, BucketPtrs B, 
   wemask[x] = static_cast<uint8_t>(bits);
 }
 
+// Node words (DevNodes), a warp per word: first the bits, row0 and the number
+// of other members, then with their exclusive sum other0 and orow.
+__global__ void k_node_words(const int32_t* __restrict__ code, const uint8_t* __restrict__ nmem, int64_t N,
+                             int64_t nwords, NodeWord* __restrict__ words, uint32_t* __restrict__ nmem_bits,
+                             int32_t* __restrict__ others) {
+  const int64_t n = static_cast<int64_t>(blockIdx.x) * kT + threadIdx.x;
+  if ((n >> 5) >= nwords) return;  // whole warps
+  const int32_t c = n < N ? code[n] : INT32_MIN;
+  const uint32_t first = __ballot_sync(0xffffffffu, c >= 0);
+  const uint32_t other = __ballot_sync(0xffffffffu, c < 0 && c != INT32_MIN);
+  const uint32_t mem = __ballot_sync(0xffffffffu, c != INT32_MIN && nmem[n]);
+  const int32_t r0 = __shfl_sync(0xffffffffu, c, first ? __ffs(first) - 1 : 0);
+  if ((threadIdx.x & 31) == 0) {
+    words[n >> 5] = NodeWord{first, other, first ? r0 : 0, 0};
+    nmem_bits[n >> 5] = mem;
+    others[n >> 5] = __popc(other);
+  }
+}
+
+__global__ void k_node_others(const int32_t* __restrict__ code, const int32_t* __restrict__ other0, int64_t N,
+                              int64_t nwords, NodeWord* __restrict__ words, int32_t* __restrict__ orow) {
+  const int64_t n = static_cast<int64_t>(blockIdx.x) * kT + threadIdx.x;
+  if ((n >> 5) >= nwords) return;
+  const int lane = threadIdx.x & 31;
+  const uint32_t other = words[n >> 5].other;
+  const int32_t o = other0[n >> 5];
+  if (lane == 0) words[n >> 5].other0 = o;
+  if ((other >> lane) & 1u) orow[o + __popc(other & ((1u << lane) - 1u))] = ~code[n];
+}
+
 // Device scratch of one setup call, freed on every exit path.
 struct Scratch {
   std::vector<void*> bufs;
@@ -381,7 +419,7 @@ cudaError_t inclusive_sum(Scratch& sc, const T* in, T* out, int64_t n, cudaStrea
 }  // namespace
 
 ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_t* ciT, const int32_t* rsN,
-                               const int32_t* ciN, void* stream) {
+                               const int32_t* ciN, const int32_t* code, const uint8_t* nmem, void* stream) {
   TraceRange trace("ogs_setup: layout on the GPU");
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   HostLayout& L = h->lay;
@@ -537,6 +575,11 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
   const size_t o_gtiles = add(L.gtiles.size() * sizeof(Tile));
   const size_t o_wtiles = add(L.wtiles.size() * sizeof(Tile));
   const size_t o_wemask = add(sgn ? L.wtiles.size() * 32 : 0);
+  const bool words = wants_node_words(h);
+  const int64_t nwords = words ? node_words(h->N) : 0;
+  const size_t o_words = add(words ? node_words_padded(h->N) * sizeof(NodeWord) : 0);
+  const size_t o_nmem = add(words ? node_words_padded(h->N) * 4 : 0);
+  const size_t o_orow = add(words ? static_cast<size_t>(h->nnzT - R) * 4 : 0);
   const size_t o_wrecs = add(L.wtiles.size() * sizeof(WarpRec));
   const size_t o_err = add(sizeof(uint32_t));  // ids out of range (checked builds); zeroed with the arena
   int dev = 0;
@@ -596,6 +639,18 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
   if (nw + ngt)
     k_tile_bounds<<<nblocks((nw + ngt) * 32), kT, 0, st>>>(d_wt, nw, B, d_gt, ngt, g_sT, g_cT, d_lo, d_hi);
   if (sgn && nw) k_wemask<<<nblocks(nw * 32), kT, 0, st>>>(d_wt, nw, B, reinterpret_cast<uint8_t*>(base + o_wemask));
+  NodeWord* d_words = reinterpret_cast<NodeWord*>(base + o_words);
+  if (words) {
+    int32_t *others = nullptr, *other0 = nullptr;
+    e = sc.get(&others, nwords);
+    if (!e) e = sc.get(&other0, nwords);
+    if (e) return release(e, "allocation");
+    k_node_words<<<nblocks(nwords * 32), kT, 0, st>>>(code, nmem, h->N, nwords, d_words,
+                                                      reinterpret_cast<uint32_t*>(base + o_nmem), others);
+    if ((e = exclusive_sum(sc, others, other0, nwords, st))) return release(e, "scan");
+    k_node_others<<<nblocks(nwords * 32), kT, 0, st>>>(code, other0, h->N, nwords, d_words,
+                                                       reinterpret_cast<int32_t*>(base + o_orow));
+  }
   std::vector<int64_t> lo(static_cast<size_t>(nw + ngt)), hi(static_cast<size_t>(nw + ngt));
   if (nw + ngt) {
     e = cudaMemcpyAsync(lo.data(), d_lo, (nw + ngt) * sizeof(int64_t), cudaMemcpyDeviceToHost, st);
@@ -638,6 +693,10 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
   m.nwtiles = static_cast<int32_t>(nw);
   m.wemask = reinterpret_cast<const uint8_t*>(base + o_wemask);
   m.wrecs = reinterpret_cast<const WarpRec*>(base + o_wrecs);
+  m.nodes.words = d_words;
+  m.nodes.nmem = reinterpret_cast<const uint32_t*>(base + o_nmem);
+  m.nodes.orow = reinterpret_cast<const int32_t*>(base + o_orow);
+  m.nodes.nwords = nwords;
   m.signed_maps = sgn ? 1 : 0;
   set_id_bounds(h, m, reinterpret_cast<unsigned int*>(base + o_err));
   return OGS_OK;
@@ -695,7 +754,15 @@ ogs_status build_device_maps(ogs_handle_s* h, int64_t N, int64_t* ids, int kind,
   e = cudaMemcpyAsync(d_ids, ids, static_cast<size_t>(N) * sizeof(int64_t), cudaMemcpyHostToDevice, st);
   if (!e) e = cudaMemsetAsync(d_c, 0, sizeof(Counters), st);
   if (e) return fail(e, "copy in");
-  k_keys<<<rblocks(N), kT, 0, st>>>(d_ids, N, key, val, d_c);
+  // whether the handle gets node words is not known yet: Signed ones may
+  int32_t* code = nullptr;
+  uint8_t* nmem = nullptr;
+  if (sgn && layout) {
+    e = sc.get(&code, N);
+    if (!e) e = sc.get(&nmem, N);
+    if (e) return fail(e, "allocation");
+  }
+  k_keys<<<rblocks(N), kT, 0, st>>>(d_ids, N, key, val, code, d_c);
   Counters c{};
   e = cudaMemcpyAsync(&c, d_c, sizeof(Counters), cudaMemcpyDeviceToHost, st);
   if (!e) e = cudaStreamSynchronize(st);
@@ -776,7 +843,8 @@ ogs_status build_device_maps(ogs_handle_s* h, int64_t N, int64_t* ids, int kind,
   k_rows<<<nblocks(ngroups), kT, 0, st>>>(gfirst, gsize, gpos, rank, ngroups, nlocalP, grow, degT, degN);
   if ((e = exclusive_sum(sc, degT, rsT, ngroups + 1, st))) return fail(e, "scan");
   if (sgn && (e = exclusive_sum(sc, degN, rsN, ngroups + 1, st))) return fail(e, "scan");
-  k_fill<<<nblocks(nnz), kT, 0, st>>>(gincl, gstart, grow, sval, pos, pos_ex, rsT, rsN, nnz, sgn ? 1 : 0, ciT, ciN);
+  k_fill<<<nblocks(nnz), kT, 0, st>>>(gincl, gstart, grow, sval, pos, pos_ex, rsT, rsN, nnz, sgn ? 1 : 0, ciT, ciN, code,
+                                     nmem);
   if (unique) k_unique_ids<<<nblocks(nnz), kT, 0, st>>>(d_ids, sval, head, nnz);
   if ((e = cudaGetLastError())) return fail(e, "kernels");
 
@@ -789,7 +857,7 @@ ogs_status build_device_maps(ogs_handle_s* h, int64_t N, int64_t* ids, int kind,
   h->nnzT = nnz;
   // the kernels' layout, built from the maps while they are on the device
   if (layout) {
-    ogs_status ls = build_device_layout(h, rsT, ciT, sgn ? rsN : nullptr, sgn ? ciN : nullptr, st);
+    ogs_status ls = build_device_layout(h, rsT, ciT, sgn ? rsN : nullptr, sgn ? ciN : nullptr, code, nmem, st);
     if (ls != OGS_OK) return ls;
   }
   // maps back to the host

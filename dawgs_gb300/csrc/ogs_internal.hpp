@@ -168,6 +168,24 @@ inline uint32_t batch_kmagic(int K) { return K > 1 && K < 11585 ? 0xFFFFFFFFu / 
 // their K components adjacent.
 
 
+// 32 consecutive nodes of a handle whose rows are numbered by first member
+// (ogs_scatter.cuh): which of them are their row's first member -- their rows
+// are row0, row0 + 1, ... -- and which another, whose rows are listed from
+// orow[other0] on.
+struct alignas(16) NodeWord {
+  uint32_t first, other;
+  int32_t row0, other0;
+};
+struct DevNodes {
+  const NodeWord* words;  // padded with empty words to a multiple of kNodeWordPad
+  const uint32_t* nmem;   // bit per node: in the N map (padded alike)
+  const int32_t* orow;
+  int64_t nwords;         // 0: the handle has none
+};
+constexpr int kNodeWordPad = 16;
+inline int64_t node_words(int64_t N) { return (N + 31) / 32; }
+inline int64_t node_words_padded(int64_t N) { return (node_words(N) + kNodeWordPad - 1) / kNodeWordPad * kNodeWordPad; }
+
 struct DevMaps {
   DevBucket b[kDmax + 1];  // b[0] unused
   DevGeneral g;
@@ -180,6 +198,7 @@ struct DevMaps {
   const uint8_t* wemask;   // [nwtiles][32] per-lane entry masks of the N map (Signed only)
   int32_t nwtiles;
   const WarpRec* wrecs;    // [nwtiles] the warp tiles as records (batched launches)
+  DevNodes nodes;
 };
 
 // Which members take part, per ogsOperator.cpp:60-97, 206-238, 311-360.
@@ -231,6 +250,9 @@ struct HostLayout {
   std::vector<Tile> gtiles;  // general CTA tiles, by first row
   std::vector<Tile> wtiles;  // exact-degree warp tiles, by first row
   std::vector<uint8_t> wemask;
+  std::vector<NodeWord> nwords;  // host path only: see DevNodes
+  std::vector<uint32_t> nmem;
+  std::vector<int32_t> orow;
   std::vector<Phase> phases;
   int64_t g_n = 0, g_nnzT = 0;  // general-bucket rows and T entries
   // lowest and highest local node each warp tile / general tile touches
@@ -288,8 +310,17 @@ void release_device(ogs_handle_s* h);
 void build_phases(ogs_handle_s* h, int max_phases);  // needs the tiles and their lo/hi
 // The maps' layout built on the current device from device CSR maps
 // (ogs_dsetup.cu): the arena, DevMaps and the host-side tile lists and phases.
+// d_code: per node its row (a first member), ~row (another member) or
+// INT32_MIN; d_nmem: per node whether it is an N member (both only read when
+// the handle gets node words).
 ogs_status build_device_layout(ogs_handle_s* h, const int32_t* d_rsT, const int32_t* d_ciT, const int32_t* d_rsN,
-                               const int32_t* d_ciN, void* stream);
+                               const int32_t* d_ciN, const int32_t* d_code, const uint8_t* d_nmem, void* stream);
+// Whether a handle gets node words: Scatter is defined and every row has a
+// positive member, so that rows are numbered by first member.
+inline bool wants_node_words(const ogs_handle_s* h) {
+  return h->kind == OGS_SIGNED && h->gather_defined && !h->from_maps && !h->gslib && h->NlocalT > 0 &&
+         h->NlocalP == h->NlocalT;
+}
 // DevMaps restricted to the tiles of one phase.
 DevMaps phase_maps(const DevMaps& m, const Phase& p);
 // The id ranges and error word of every bucket (both setup paths).

@@ -1,8 +1,9 @@
 // ogs_launch.cuh -- per-type launch dispatch shared by ogs_kern_*.cu.
 //
-// Exact-degree rows of GatherScatter run on the warp pipeline with
-// cp.async-staged gathers (ogs_async.cuh), those of Gather and Scatter on the
-// register pipeline of ogs_warp.cuh (-DOGS_GATHER_REGISTERS=0: everything on
+// Scatter runs in node order where the handle's rows are numbered by first
+// member (ogs_scatter.cuh).  Otherwise exact-degree rows of GatherScatter run
+// on the warp pipeline with cp.async-staged gathers (ogs_async.cuh), those of
+// Gather and Scatter on the register pipeline of ogs_warp.cuh (-DOGS_GATHER_REGISTERS=0: everything on
 // the cp.async one; -DOGS_ASYNC=0: everything on the register one).  Rows
 // above degree 8 run on the direct CTA kernel (ogs_kernels.cuh).  Building
 // with -DOGS_KERNEL=2 runs the direct CTA kernel for every row instead (for
@@ -18,6 +19,7 @@
 #pragma once
 
 #include "ogs_async.cuh"
+#include "ogs_scatter.cuh"
 
 #ifndef OGS_KERNEL
 #define OGS_KERNEL 0
@@ -57,6 +59,7 @@ inline int launch_typed(const DevMaps& m, const FieldArgs& f, int mode, int op, 
   cudaError_t e;
   if (mode == kModeGS) e = launch_op<T, kModeGS>(m, f, op, pat, s);
   else if (mode == kModeGather) e = launch_op<T, kModeGather>(m, f, op, pat, s);
+  else if (OGS_KERNEL == 0 && scatter_applies(m, f, pat)) e = launch_scatter<T>(m, f, pat, s);
   else e = launch_mode<T, OGS_ADD, kModeScatter>(m, f, pat, s);  // a copy: op unused
   return static_cast<int>(e);
 }

@@ -297,6 +297,32 @@ void build_layout(ogs_handle_s* h) {
   }
   L.tiles.insert(L.tiles.end(), L.gtiles.begin(), L.gtiles.end());
   std::stable_sort(L.tiles.begin(), L.tiles.end(), by_row);
+  L.nwords.clear();
+  L.nmem.clear();
+  L.orow.clear();
+  if (wants_node_words(h)) {
+    std::vector<int32_t> rowof(static_cast<size_t>(h->N), -1);
+    L.nwords.assign(node_words_padded(h->N), NodeWord{0, 0, 0, 0});
+    L.nmem.assign(L.nwords.size(), 0);
+    for (int64_t r = 0; r < R; ++r) {
+      for (int32_t q = rsT[r]; q < rsT[r + 1]; ++q) rowof[ciT[q]] = static_cast<int32_t>(r);
+      for (int32_t q = rsN[r]; q < rsN[r + 1]; ++q) L.nmem[ciN[q] >> 5] |= 1u << (ciN[q] & 31);
+    }
+    L.orow.reserve(h->nnzT - R);
+    for (int64_t n = 0; n < h->N; ++n) {
+      NodeWord& w = L.nwords[n >> 5];
+      const int32_t r = rowof[n];
+      if ((n & 31) == 0) w.other0 = static_cast<int32_t>(L.orow.size());
+      if (r < 0) continue;
+      if (ciT[rsT[r]] == n) {
+        if (!w.first) w.row0 = r;
+        w.first |= 1u << (n & 31);
+      } else {
+        w.other |= 1u << (n & 31);
+        L.orow.push_back(r);
+      }
+    }
+  }
   L.g_n = static_cast<int64_t>(L.g_rows.size());
   L.g_nnzT = static_cast<int64_t>(L.g_colsT.size());
   // lowest and highest node of every tile (the host pipeline's slices)
@@ -452,8 +478,11 @@ void set_id_bounds(const ogs_handle_s* h, DevMaps& m, unsigned int* err) {
   m.g.err = err;
 }
 
+// A slice runs on its tiles alone: they say which nodes it touches, and the
+// copies of a sliced host-buffer call set its time.
 DevMaps phase_maps(const DevMaps& m, const Phase& p) {
   DevMaps r = m;
+  r.nodes.nwords = 0;
   r.wtiles = m.wtiles + p.w0;
   r.nwtiles = p.w1 - p.w0;
   if (m.wemask) r.wemask = m.wemask + static_cast<int64_t>(p.w0) * 32;
@@ -508,6 +537,9 @@ ogs_status upload_layout(ogs_handle_s* h) {
   const size_t o_gtiles = add(L.gtiles.data(), L.gtiles.size() * sizeof(Tile));
   const size_t o_wtiles = add(L.wtiles.data(), L.wtiles.size() * sizeof(Tile));
   const size_t o_wemask = add(L.wemask.data(), L.wemask.size());
+  const size_t o_words = add(L.nwords.data(), L.nwords.size() * sizeof(NodeWord));
+  const size_t o_nmem = add(L.nmem.data(), L.nmem.size() * 4);
+  const size_t o_orow = add(L.orow.data(), L.orow.size() * 4);
   // warp records hold device pointers: filled in once the arena exists
   std::vector<WarpRec> wrecs(L.wtiles.size());
   const size_t o_wrecs = add(wrecs.data(), wrecs.size() * sizeof(WarpRec));
@@ -570,6 +602,10 @@ ogs_status upload_layout(ogs_handle_s* h) {
   m.nwtiles = static_cast<int32_t>(L.wtiles.size());
   m.wemask = reinterpret_cast<const uint8_t*>(base + o_wemask);
   m.wrecs = reinterpret_cast<const WarpRec*>(base + o_wrecs);
+  m.nodes.words = reinterpret_cast<const NodeWord*>(base + o_words);
+  m.nodes.nmem = reinterpret_cast<const uint32_t*>(base + o_nmem);
+  m.nodes.orow = reinterpret_cast<const int32_t*>(base + o_orow);
+  m.nodes.nwords = L.nwords.empty() ? 0 : node_words(h->N);
   set_id_bounds(h, m, reinterpret_cast<unsigned int*>(base + o_err));
 
   m.signed_maps = sgn ? 1 : 0;
