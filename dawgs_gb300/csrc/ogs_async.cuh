@@ -325,7 +325,7 @@ inline void launch_async_kl(const DevMaps& m, const FieldArgs& f, Pattern pat, c
   }
 }
 
-// Exact-degree tiles on the async pipeline, general tiles on the direct kernel.
+// Exact-degree tiles on the async pipeline, general rows in a launch of their own.
 template <typename T, int OP, int MODE>
 inline cudaError_t launch_async(const DevMaps& m, const FieldArgs& f, Pattern pat, cudaStream_t s) {
   if (m.nwtiles > 0) {
@@ -335,13 +335,7 @@ inline cudaError_t launch_async(const DevMaps& m, const FieldArgs& f, Pattern pa
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  if (m.ngtiles > 0) {
-    DevMaps g = m;
-    g.tiles = m.gtiles;
-    g.ntiles = m.ngtiles;
-    return launch_direct<T, OP, MODE>(g, f, pat, s);
-  }
-  return cudaSuccess;
+  return launch_general<T, OP, MODE>(m, f, pat, s);
 }
 
 }  // namespace ogsgb

@@ -107,11 +107,7 @@ ogs_status apply_config(ogs_batch_s* b, const BatchEntry* fields, cudaStream_t s
 
 int launch_typed_entry(int type, const ogs_handle_s* h, void* v, int k, int op, const BatchEntry& be, bool general_only,
                        cudaStream_t st) {
-  DevMaps m = h->dmaps;
-  if (general_only) {
-    m.nwtiles = 0;
-    m.ntiles = m.ngtiles;
-  }
+  const DevMaps m = general_only ? general_maps(h->dmaps) : h->dmaps;
   FieldArgs f{};
   f.v = v;
   f.K = k;

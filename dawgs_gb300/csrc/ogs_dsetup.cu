@@ -349,6 +349,30 @@ __global__ void k_wemask(const Tile* __restrict__ wt, int64_t nw, BucketPtrs B, 
   wemask[x] = static_cast<uint8_t>(bits);
 }
 
+// Ids of the wide tiles (DevMaps::wide), a warp per tile.
+__global__ void k_wide_ids(const Tile* __restrict__ wide, int64_t nwide, const int32_t* __restrict__ startsT,
+                           const int32_t* __restrict__ colsT, const int32_t* __restrict__ startsN,
+                           const int32_t* __restrict__ colsN, uint32_t* __restrict__ ids) {
+  const int64_t t = (static_cast<int64_t>(blockIdx.x) * kT + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (t >= nwide) return;
+  const Tile w = wide[t];
+  const int64_t u0 = static_cast<int64_t>(w.first_row) * 32;
+  for (int i = lane; i < w.bucket * 32; i += 32) ids[u0 + i] = kNoWideId;
+  __syncwarp();
+  if (lane >= w.count) return;  // a lane a row
+  const int32_t s = startsT[w.begin + lane], d = startsT[w.begin + lane + 1] - s;
+  int32_t n = startsN[w.begin + lane];
+  const int32_t ne = startsN[w.begin + lane + 1];
+  for (int q = 0; q < d; ++q) {
+    const int32_t c = colsT[s + q];
+    // N members are a subsequence of the T members
+    const bool member = n < ne && colsN[n] == c;
+    if (member) ++n;
+    ids[u0 + q * 32 + lane] = static_cast<uint32_t>(c) | (member ? 0x80000000u : 0u);
+  }
+}
+
 // Node words (DevNodes), a warp per word: first the bits, row0 and the number
 // of other members, then with their exclusive sum other0 and orow.
 __global__ void k_node_words(const int32_t* __restrict__ code, const uint8_t* __restrict__ nmem, int64_t N,
@@ -575,6 +599,9 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
   const size_t o_gtiles = add(L.gtiles.size() * sizeof(Tile));
   const size_t o_wtiles = add(L.wtiles.size() * sizeof(Tile));
   const size_t o_wemask = add(sgn ? L.wtiles.size() * 32 : 0);
+  const int64_t wide_units = wide_layout(g_startsT.data(), ng, L.wide);
+  const size_t o_wide = add(L.wide.size() * sizeof(Tile));
+  const size_t o_wids = add(static_cast<size_t>(wide_units) * 32 * 4);
   const bool words = wants_node_words(h);
   const int64_t nwords = words ? node_words(h->N) : 0;
   const size_t o_words = add(words ? node_words_padded(h->N) * sizeof(NodeWord) : 0);
@@ -630,7 +657,12 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
   if (!e) e = cudaMemcpyAsync(base + o_gtiles, L.gtiles.data(), L.gtiles.size() * sizeof(Tile), cudaMemcpyHostToDevice, st);
   if (!e) e = cudaMemcpyAsync(base + o_wtiles, L.wtiles.data(), L.wtiles.size() * sizeof(Tile), cudaMemcpyHostToDevice, st);
   if (!e) e = cudaMemcpyAsync(base + o_wrecs, wrecs.data(), wrecs.size() * sizeof(WarpRec), cudaMemcpyHostToDevice, st);
+  Tile* d_wide = reinterpret_cast<Tile*>(base + o_wide);
+  uint32_t* d_wids = reinterpret_cast<uint32_t*>(base + o_wids);
+  const int64_t nwide = static_cast<int64_t>(L.wide.size());
+  if (!e && nwide) e = cudaMemcpyAsync(d_wide, L.wide.data(), nwide * sizeof(Tile), cudaMemcpyHostToDevice, st);
   if (e) return release(e, "tiles");
+  if (nwide) k_wide_ids<<<nblocks(nwide * 32), kT, 0, st>>>(d_wide, nwide, g_sT, g_cT, g_sN, g_cN, d_wids);
   const int64_t ngt = static_cast<int64_t>(L.gtiles.size());
   int64_t *d_lo = nullptr, *d_hi = nullptr;
   e = sc.get(&d_lo, nw + ngt);
@@ -693,6 +725,9 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
   m.nwtiles = static_cast<int32_t>(nw);
   m.wemask = reinterpret_cast<const uint8_t*>(base + o_wemask);
   m.wrecs = reinterpret_cast<const WarpRec*>(base + o_wrecs);
+  m.wide = d_wide;
+  m.wide_ids = d_wids;
+  m.nwide = static_cast<int32_t>(nwide);
   m.nodes.words = d_words;
   m.nodes.nmem = reinterpret_cast<const uint32_t*>(base + o_nmem);
   m.nodes.orow = reinterpret_cast<const int32_t*>(base + o_orow);

@@ -186,6 +186,10 @@ constexpr int kNodeWordPad = 16;
 inline int64_t node_words(int64_t N) { return (N + 31) / 32; }
 inline int64_t node_words_padded(int64_t N) { return (node_words(N) + kNodeWordPad - 1) / kNodeWordPad * kNodeWordPad; }
 
+// Member of a wide tile's row: node | N member << 31, or none.
+constexpr uint32_t kNoWideId = 0xFFFFFFFFu;
+constexpr int kWideRows = 32;  // rows of a wide tile
+
 struct DevMaps {
   DevBucket b[kDmax + 1];  // b[0] unused
   DevGeneral g;
@@ -199,6 +203,12 @@ struct DevMaps {
   int32_t nwtiles;
   const WarpRec* wrecs;    // [nwtiles] the warp tiles as records (batched launches)
   DevNodes nodes;
+  // The general rows, kWideRows a tile (ogs_wide.cuh): bucket = the longest
+  // row's degree, begin and count in the general bucket, member q of the
+  // tile's row j at wide_ids[(first_row + q) * 32 + j].
+  const Tile* wide;
+  const uint32_t* wide_ids;
+  int32_t nwide;           // 0: the general rows run as CTA tiles
 };
 
 // Which members take part, per ogsOperator.cpp:60-97, 206-238, 311-360.
@@ -253,6 +263,8 @@ struct HostLayout {
   std::vector<NodeWord> nwords;  // host path only: see DevNodes
   std::vector<uint32_t> nmem;
   std::vector<int32_t> orow;
+  std::vector<Tile> wide;          // see DevMaps
+  std::vector<uint32_t> wide_ids;  // host path only
   std::vector<Phase> phases;
   int64_t g_n = 0, g_nnzT = 0;  // general-bucket rows and T entries
   // lowest and highest local node each warp tile / general tile touches
@@ -321,6 +333,12 @@ inline bool wants_node_words(const ogs_handle_s* h) {
   return h->kind == OGS_SIGNED && h->gather_defined && !h->from_maps && !h->gslib && h->NlocalT > 0 &&
          h->NlocalP == h->NlocalT;
 }
+// Wide tiles of general rows with the given row starts; the units of 32 ids
+// they take.  None where rows of very different degree are neighbours and the
+// padding would outweigh the rows.
+int64_t wide_layout(const int32_t* starts, int64_t rows, std::vector<Tile>& wide);
+// DevMaps restricted to the general rows.
+DevMaps general_maps(const DevMaps& m);
 // DevMaps restricted to the tiles of one phase.
 DevMaps phase_maps(const DevMaps& m, const Phase& p);
 // The id ranges and error word of every bucket (both setup paths).

@@ -26,6 +26,20 @@
 
 namespace ogsgb {
 
+// How the k components of a field map onto work items.
+enum KLayout : int {
+  kK1 = 0,          // k = 1: item = tile
+  kKInterleaved = 1,  // v[c + n*k], k > 1: item = (tile, part), tile-major;
+                      // part j takes the tile's (row lane, component) units
+                      // 32j .. 32j+31, so neighbouring threads read the k
+                      // values of one node in one instruction.  (One item per
+                      // tile looping over the components was slower: 86 vs
+                      // 66 us for k = 3 on 3.5 M permuted nodes.)
+  kKMany = 2,       // k separate arrays: item = (array, tile), array-major, so
+                    // one array and the column ids stay resident in L2 while
+                    // the grid sweeps that array
+};
+
 // A column or row id loaded from the maps, checked against [0, lim) in
 // checked builds: an id outside is counted in *err and replaced by 0.
 __device__ __forceinline__ int32_t checked_id(int32_t id, int32_t lim, unsigned int* err) {

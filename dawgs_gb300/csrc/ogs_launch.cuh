@@ -3,9 +3,10 @@
 // Scatter runs in node order where the handle's rows are numbered by first
 // member (ogs_scatter.cuh).  Otherwise exact-degree rows of GatherScatter run
 // on the warp pipeline with cp.async-staged gathers (ogs_async.cuh), those of
-// Gather and Scatter on the register pipeline of ogs_warp.cuh (-DOGS_GATHER_REGISTERS=0: everything on
-// the cp.async one; -DOGS_ASYNC=0: everything on the register one).  Rows
-// above degree 8 run on the direct CTA kernel (ogs_kernels.cuh).  Building
+// Gather and Scatter on the register pipeline of ogs_warp.cuh
+// (-DOGS_GATHER_REGISTERS=0: everything on the cp.async one; -DOGS_ASYNC=0:
+// everything on the register one).  Rows above degree 8 run as wide tiles
+// (ogs_wide.cuh), or on the direct CTA kernel (ogs_kernels.cuh).  Building
 // with -DOGS_KERNEL=2 runs the direct CTA kernel for every row instead (for
 // comparisons).
 //

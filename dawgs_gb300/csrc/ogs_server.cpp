@@ -227,9 +227,7 @@ int batch_launch(int type, const BatchEntry* E, const int64_t* starts, int n, in
 }
 
 int general_launch(int type, const ogs_handle_s* h, void* v, int k, int op, const Pattern& pat, cudaStream_t st) {
-  DevMaps g = h->dmaps;
-  g.nwtiles = 0;
-  g.ntiles = g.ngtiles;
+  const DevMaps g = general_maps(h->dmaps);
   FieldArgs f{};
   f.v = v;
   f.K = k;

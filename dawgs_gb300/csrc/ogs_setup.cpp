@@ -181,6 +181,24 @@ ogs_status build_host_maps(ogs_handle_s* h, int64_t N, int64_t* ids, int kind, i
   return OGS_OK;
 }
 
+int64_t wide_layout(const int32_t* starts, int64_t rows, std::vector<Tile>& wide) {
+  wide.clear();
+  int64_t units = 0;
+  for (int64_t i = 0; i < rows; i += kWideRows) {
+    const int64_t n = std::min<int64_t>(kWideRows, rows - i);
+    int32_t d = 0;
+    for (int64_t j = i; j < i + n; ++j) d = std::max(d, starts[j + 1] - starts[j]);
+    wide.push_back(Tile{d, static_cast<int32_t>(i), static_cast<int32_t>(n), static_cast<int32_t>(units)});
+    units += d;
+  }
+  // an odd last tile alone may be mostly padding: 2048 ids more than twice the rows'
+  if (units * 32 > 2 * static_cast<int64_t>(starts[rows]) + 2048) {
+    wide.clear();
+    units = 0;
+  }
+  return units;
+}
+
 void build_layout(ogs_handle_s* h) {
   TraceRange trace("ogs_setup: layout on the host");
   HostLayout& L = h->lay;
@@ -297,6 +315,24 @@ void build_layout(ogs_handle_s* h) {
   }
   L.tiles.insert(L.tiles.end(), L.gtiles.begin(), L.gtiles.end());
   std::stable_sort(L.tiles.begin(), L.tiles.end(), by_row);
+  L.wide.clear();
+  L.wide_ids.clear();
+  if (!h->gslib) {
+    const int64_t units = wide_layout(L.g_startsT.data(), static_cast<int64_t>(L.g_rows.size()), L.wide);
+    L.wide_ids.assign(static_cast<size_t>(units) * 32, kNoWideId);
+    for (const Tile& w : L.wide)
+      for (int32_t j = 0; j < w.count; ++j) {
+        const int32_t i = w.begin + j;
+        int32_t n = L.g_startsN[i];
+        for (int32_t q = 0; q < L.g_startsT[i + 1] - L.g_startsT[i]; ++q) {
+          const int32_t c = L.g_colsT[L.g_startsT[i] + q];
+          const bool member = n < L.g_startsN[i + 1] && L.g_colsN[n] == c;
+          if (member) ++n;
+          L.wide_ids[(static_cast<size_t>(w.first_row) + q) * 32 + j] =
+              static_cast<uint32_t>(c) | (member ? 0x80000000u : 0u);
+        }
+      }
+  }
   L.nwords.clear();
   L.nmem.clear();
   L.orow.clear();
@@ -478,11 +514,19 @@ void set_id_bounds(const ogs_handle_s* h, DevMaps& m, unsigned int* err) {
   m.g.err = err;
 }
 
+DevMaps general_maps(const DevMaps& m) {
+  DevMaps g = m;
+  g.nwtiles = 0;
+  g.ntiles = g.ngtiles;
+  return g;
+}
+
 // A slice runs on its tiles alone: they say which nodes it touches, and the
 // copies of a sliced host-buffer call set its time.
 DevMaps phase_maps(const DevMaps& m, const Phase& p) {
   DevMaps r = m;
   r.nodes.nwords = 0;
+  r.nwide = 0;
   r.wtiles = m.wtiles + p.w0;
   r.nwtiles = p.w1 - p.w0;
   if (m.wemask) r.wemask = m.wemask + static_cast<int64_t>(p.w0) * 32;
@@ -537,6 +581,8 @@ ogs_status upload_layout(ogs_handle_s* h) {
   const size_t o_gtiles = add(L.gtiles.data(), L.gtiles.size() * sizeof(Tile));
   const size_t o_wtiles = add(L.wtiles.data(), L.wtiles.size() * sizeof(Tile));
   const size_t o_wemask = add(L.wemask.data(), L.wemask.size());
+  const size_t o_wide = add(L.wide.data(), L.wide.size() * sizeof(Tile));
+  const size_t o_wids = add(L.wide_ids.data(), L.wide_ids.size() * 4);
   const size_t o_words = add(L.nwords.data(), L.nwords.size() * sizeof(NodeWord));
   const size_t o_nmem = add(L.nmem.data(), L.nmem.size() * 4);
   const size_t o_orow = add(L.orow.data(), L.orow.size() * 4);
@@ -602,6 +648,9 @@ ogs_status upload_layout(ogs_handle_s* h) {
   m.nwtiles = static_cast<int32_t>(L.wtiles.size());
   m.wemask = reinterpret_cast<const uint8_t*>(base + o_wemask);
   m.wrecs = reinterpret_cast<const WarpRec*>(base + o_wrecs);
+  m.wide = reinterpret_cast<const Tile*>(base + o_wide);
+  m.wide_ids = reinterpret_cast<const uint32_t*>(base + o_wids);
+  m.nwide = static_cast<int32_t>(L.wide.size());
   m.nodes.words = reinterpret_cast<const NodeWord*>(base + o_words);
   m.nodes.nmem = reinterpret_cast<const uint32_t*>(base + o_nmem);
   m.nodes.orow = reinterpret_cast<const int32_t*>(base + o_orow);

@@ -29,7 +29,7 @@
 
 #include <cstdint>
 
-#include "ogs_kernels.cuh"
+#include "ogs_wide.cuh"
 
 // Minimum resident CTAs per SM the register allocation must allow.
 #ifndef OGS_WARP_MINB
@@ -161,20 +161,6 @@ __device__ __forceinline__ void warp_fold_store(const WarpState& s, T* dst, T* g
     default: CALL(8); break;            \
   }
 
-// How the k components of a field map onto work items.
-enum KLayout : int {
-  kK1 = 0,          // k = 1: item = tile
-  kKInterleaved = 1,  // v[c + n*k], k > 1: item = (tile, part), tile-major;
-                      // part j takes the tile's (row lane, component) units
-                      // 32j .. 32j+31, so neighbouring threads read the k
-                      // values of one node in one instruction.  (One item per
-                      // tile looping over the components was slower: 86 vs
-                      // 66 us for k = 3 on 3.5 M permuted nodes.)
-  kKMany = 2,       // k separate arrays: item = (array, tile), array-major, so
-                    // one array and the column ids stay resident in L2 while
-                    // the grid sweeps that array
-};
-
 template <typename T, int OP, int MODE, int KL, bool PLAIN>
 __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_warp_kernel(const DevMaps m, const FieldArgs f,
                                                                          const Pattern pat_in) {
@@ -294,13 +280,7 @@ inline cudaError_t launch_warp(const DevMaps& m, const FieldArgs& f, Pattern pat
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
-  if (m.ngtiles > 0) {
-    DevMaps g = m;
-    g.tiles = m.gtiles;
-    g.ntiles = m.ngtiles;
-    return launch_direct<T, OP, MODE>(g, f, pat, s);
-  }
-  return cudaSuccess;
+  return launch_general<T, OP, MODE>(m, f, pat, s);
 }
 
 }  // namespace ogsgb

@@ -1,0 +1,114 @@
+// ogs_wide.cuh -- rows above degree 8, a lane a row.
+//
+// The reference folds such a row like any other (ogsOperator.cpp:60-97,
+// 206-238, 311-360), in ascending member order.  What bounds it is latency and
+// the requests of members that lie in as many sectors.  The column ids of 32
+// consecutive rows are laid out member by member (a coalesced load each), a
+// lane has up to 24 members in flight, and k components are split over a
+// tile's k parts as in ogs_async.cuh.  Before, a CTA took up to 256 rows
+// through their CSR lists, a thread a row and one load after the other, all
+// components in turn.  GatherScatter fp64, vertices of degree 24, us a call
+// before and now: 64^3 cells of six p=1 tetrahedra 69.8 -> 58.5, 20x20x16 of
+// p=3 with k=3 27.8 -> 17.0, 24^3 of p=2 in 4 arrays 43.8 -> 32.4, 32x32x24 of
+// p=3 27.3 -> 26.2.  Slower forms: four lanes a row with the members passed by
+// shuffles (an fp64 add costs a warp 16 cycles of its pipe whatever lanes take
+// part), and the tiles at the head of the launch of the exact-degree rows (28-34
+// us in the last case, and that kernel 3 % slower where there are none).
+#pragma once
+
+#include <algorithm>
+#include <cstdint>
+
+#include "ogs_kernels.cuh"
+
+namespace ogsgb {
+
+constexpr int kWideBatch = 24;  // members a lane has in flight
+constexpr int kWideBlock = 64;  // small CTAs, so that a few hundred tiles reach every SM
+
+// One work item: component k of row rl of wide tile `t`.
+template <typename T, int OP, int MODE>
+__device__ __forceinline__ void wide_tile(const DevMaps& m, const FieldArgs& f, const Pattern& pat, int t, int rl,
+                                          int k, int K, int64_t stride) {
+  constexpr int B = kWideBatch;
+  const Tile w = m.wide[t];
+  if (rl >= w.count || (pat.limit_n && w.begin + rl >= m.g.nP)) return;
+  const uint32_t* ids = m.wide_ids + static_cast<int64_t>(w.first_row) * 32 + rl;
+  const int d = w.bucket;
+  const int64_t r = MODE == kModeGS ? 0 : checked_id(__ldg(m.g.rows + w.begin + rl), m.g.nrows, m.g.err);
+  T a;
+  if (MODE == kModeScatter) {
+    a = static_cast<const T*>(f.gv)[r * K + k];
+  } else {
+    const T* src = field_base<T>(f, k);
+    a = op_init<T, OP>();
+    for (int q0 = 0; q0 < d; q0 += B) {
+      uint32_t id[B];
+      T x[B];
+#pragma unroll
+      for (int q = 0; q < B; ++q) id[q] = q0 + q < d ? __ldg(ids + (q0 + q) * 32) : kNoWideId;
+#pragma unroll
+      for (int q = 0; q < B; ++q) {
+        if (pat.gather_n && !(id[q] >> 31)) id[q] = kNoWideId;
+        if (id[q] != kNoWideId)
+          x[q] = src[static_cast<int64_t>(checked_id(id[q] & 0x7FFFFFFFu, m.g.nnodes, m.g.err)) * stride];
+      }
+#pragma unroll
+      for (int q = 0; q < B; ++q)
+        if (id[q] != kNoWideId) op_apply<T, OP>(a, x[q]);
+    }
+  }
+  if (MODE == kModeGather) {
+    static_cast<T*>(f.gv)[r * K + k] = a;
+  } else {
+    T* dst = field_base<T>(f, k);
+#pragma unroll 8
+    for (int q = 0; q < d; ++q) {
+      const uint32_t id = __ldg(ids + q * 32);
+      if (id != kNoWideId && (!pat.scatter_n || (id >> 31)))
+        dst[static_cast<int64_t>(checked_id(id & 0x7FFFFFFFu, m.g.nnodes, m.g.err)) * stride] = a;
+    }
+  }
+}
+
+// All wide tiles: a warp an item, (tile, part) or (array, tile); see KLayout for
+// the parts of k > 1 interleaved.
+template <typename T, int OP, int MODE, int KL>
+__global__ void __launch_bounds__(kWideBlock) ogs_wide_kernel(const DevMaps m, const FieldArgs f, const Pattern pat) {
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  const int K = KL == kK1 ? 1 : f.K;
+  const int64_t n = static_cast<int64_t>(m.nwide) * K;
+  const int64_t W = static_cast<int64_t>(gridDim.x) * (kWideBlock / 32);
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * (kWideBlock / 32) + (threadIdx.x >> 5); i < n; i += W) {
+    if (KL == kKInterleaved) {
+      const int64_t t = i / K;
+      const uint32_t u = static_cast<uint32_t>(i - t * K) * 32u + static_cast<uint32_t>(lane);
+      const uint32_t rl = u / static_cast<uint32_t>(K);
+      wide_tile<T, OP, MODE>(m, f, pat, static_cast<int>(t), static_cast<int>(rl), static_cast<int>(u - rl * K), K, K);
+    } else {
+      const int64_t a = KL == kKMany ? i / m.nwide : 0;
+      wide_tile<T, OP, MODE>(m, f, pat, static_cast<int>(i - a * m.nwide), lane, static_cast<int>(a), K, 1);
+    }
+  }
+}
+
+// The general rows of a call: as wide tiles or, for handles without them and
+// gslib's rules, on the direct kernel.
+template <typename T, int OP, int MODE>
+inline cudaError_t launch_general(const DevMaps& m, const FieldArgs& f, Pattern pat, cudaStream_t s) {
+  if (m.ngtiles == 0) return cudaSuccess;
+  if (m.nwide == 0 || pat.gslib || pat.scatter_n > 1) {
+    DevMaps g = m;
+    g.tiles = m.gtiles;
+    g.ntiles = m.ngtiles;
+    return launch_direct<T, OP, MODE>(g, f, pat, s);
+  }
+  const int64_t n = (static_cast<int64_t>(m.nwide) * f.K + kWideBlock / 32 - 1) / (kWideBlock / 32);
+  const unsigned grid = static_cast<unsigned>(std::min<int64_t>(n, 1 << 20));
+  if (f.is_many) ogs_wide_kernel<T, OP, MODE, kKMany><<<grid, kWideBlock, 0, s>>>(m, f, pat);
+  else if (f.K == 1) ogs_wide_kernel<T, OP, MODE, kK1><<<grid, kWideBlock, 0, s>>>(m, f, pat);
+  else ogs_wide_kernel<T, OP, MODE, kKInterleaved><<<grid, kWideBlock, 0, s>>>(m, f, pat);
+  return cudaGetLastError();
+}
+
+}  // namespace ogsgb
