@@ -141,6 +141,10 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_async_kernel(const 
   // slower: 83 vs 62 us for k = 3 on 3.5 M permuted nodes.)  Items are
   // followed as (tile, part) pairs, advanced by W without division.
   const int64_t i0 = wid;
+  // The plain builds read descriptors and column ids before they wait for the
+  // work ahead (grid_wait); in the others the wait among them costs spills.
+  grid_release();
+  if (!PLAIN || i0 >= nitems) grid_wait();
   if (i0 >= nitems) return;
   int64_t i = i0;
   const int64_t step = W, iend = nitems;
@@ -219,6 +223,7 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_async_kernel(const 
     OGS_DEGREE_SWITCH(nxt.bucket, OGS_A_LOAD_NXT)
 #undef OGS_A_LOAD_NXT
   }
+  if (PLAIN) grid_wait();  // the first access to the field follows
   {
     const T* src = (MODE == kModeScatter) ? nullptr : field_base<T>(f, kcur);
 #define OGS_A_ISSUE0(D) async_issue_vals<T, MODE, D>(scur, src, gv, stride, K, kcur, gmask, rcur, lane, ring)
@@ -318,10 +323,10 @@ inline void launch_async_kl(const DevMaps& m, const FieldArgs& f, Pattern pat, c
   const bool plain = !pat.gather_n && !pat.scatter_n && !pat.limit_n && !pat.gslib;
   if (plain) {
     const int grid = async_grid<T, OP, MODE, KL, true>(nitems);
-    ogs_async_kernel<T, OP, MODE, KL, true><<<grid, kBlock, async_smem_bytes<T>(), s>>>(m, f, pat);
+    launch_overlapped(ogs_async_kernel<T, OP, MODE, KL, true>, grid, kBlock, async_smem_bytes<T>(), s, f.overlap, m, f, pat);
   } else {
     const int grid = async_grid<T, OP, MODE, KL, false>(nitems);
-    ogs_async_kernel<T, OP, MODE, KL, false><<<grid, kBlock, async_smem_bytes<T>(), s>>>(m, f, pat);
+    launch_overlapped(ogs_async_kernel<T, OP, MODE, KL, false>, grid, kBlock, async_smem_bytes<T>(), s, f.overlap, m, f, pat);
   }
 }
 

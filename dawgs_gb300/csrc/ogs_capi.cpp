@@ -97,6 +97,22 @@ ogs_status launch(const ogs_handle_s* h, const FieldArgs& f, int mode, int op, P
   return launch_maps(h->dmaps, f, mode, op, pat, type, stream, fn);
 }
 
+// Whether a call's kernel may start before the work ahead of it in the stream
+// has ended (FieldArgs::overlap).  Not while the stream is captured, so that
+// graphs hold plain kernel nodes; and not for handles with general rows, whose
+// calls are two launches: the small CTAs of one take the places that the
+// persistent CTAs of the next call's other need (gs of 32x32x24 cells of six p=3
+// tetrahedra: copy and four calls 151 us overlapped, 128 not).
+int may_overlap(const ogs_handle_s* h, void* stream) {
+  if (h->dmaps.ngtiles > 0) return 0;
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &c) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return c == cudaStreamCaptureStatusNone;
+}
+
 ogs_status ensure_stage(ogs_handle_s* h, size_t bytes, const char* fn) {
   if (bytes <= h->stage_bytes) return OGS_OK;
   if (h->stage) dev_free(h->stage);
@@ -301,6 +317,7 @@ ogs_status ogs_gather_scatter(ogs_handle h, void* d_v, int k, int type, int op, 
   FieldArgs f{};
   f.v = d_v;
   f.K = k;
+  f.overlap = may_overlap(h, stream);
   return launch(h, f, kModeGS, op, pattern_for(h, kModeGS, trans), type, stream, fn);
 }
 
@@ -317,6 +334,7 @@ ogs_status ogs_gather_scatter_many(ogs_handle h, void* const* d_vs, int k, int t
   for (int k0 = 0; k0 < k; k0 += kMaxMany) {
     FieldArgs f{};
     f.is_many = 1;
+    f.overlap = may_overlap(h, stream);
     f.K = (k - k0 < kMaxMany) ? (k - k0) : kMaxMany;
     for (int j = 0; j < f.K; ++j) {
       if (!d_vs[k0 + j]) return set_error(OGS_EINVAL, "ogs_gather_scatter_many: a field pointer is NULL");
@@ -342,6 +360,7 @@ ogs_status ogs_gather(ogs_handle h, void* d_gv, const void* d_v, int k, int type
   f.v = const_cast<void*>(d_v);
   f.gv = d_gv;
   f.K = k;
+  f.overlap = may_overlap(h, stream);
   return launch(h, f, kModeGather, op, pattern_for(h, kModeGather, trans), type, stream, fn);
 }
 
@@ -358,6 +377,7 @@ ogs_status ogs_scatter(ogs_handle h, void* d_v, const void* d_gv, int k, int typ
   f.v = d_v;
   f.gv = const_cast<void*>(d_gv);
   f.K = k;
+  f.overlap = may_overlap(h, stream);
   return launch(h, f, kModeScatter, OGS_ADD, pattern_for(h, kModeScatter, trans), type, stream, fn);
 }
 

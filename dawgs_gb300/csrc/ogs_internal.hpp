@@ -231,6 +231,7 @@ struct FieldArgs {
   void* many[kMaxMany];     // separate arrays (GS many)
   int32_t K;
   int32_t is_many;
+  int32_t overlap = 0;      // host: launch with programmatic stream serialization
 };
 
 // A slice of the warp and general tiles for the host-buffer pipeline: its

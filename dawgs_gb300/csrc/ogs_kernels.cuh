@@ -40,6 +40,33 @@ enum KLayout : int {
                     // the grid sweeps that array
 };
 
+// Programmatic dependent launch.  A call's kernels let the next one in the
+// stream start as their CTAs leave (grid_release) and, before they touch a
+// field, wait for the work before them (grid_wait: whole grids, their writes
+// visible); until then they read maps only, which do not change after setup.
+// Both are nothing for kernels launched without the attribute.  It hides the
+// gap between launches and the first two of a call's three chained loads: 24^3
+// p=7 fp64 copy and four GatherScatters 116.5 -> 109.0 us, Scatter then Gather
+// 49.8 -> 43.4, 23x19x17 p=6 int64 copy and Max 24.6 -> 22.3.
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
+template <typename... P, typename... A>
+inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t s,
+                                     bool overlap, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(static_cast<unsigned>(block));
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = overlap ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // A column or row id loaded from the maps, checked against [0, lim) in
 // checked builds: an id outside is counted in *err and replaced by 0.
 __device__ __forceinline__ int32_t checked_id(int32_t id, int32_t lim, unsigned int* err) {

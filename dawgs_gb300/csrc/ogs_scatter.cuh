@@ -38,7 +38,11 @@ __global__ void __launch_bounds__(kScatterBlock) ogs_scatter_kernel(const DevNod
   constexpr int B = KC ? KC : 8;  // runs of a word in flight
   const int lane = static_cast<int>(threadIdx.x) & 31;
   const int64_t w0 = (static_cast<int64_t>(blockIdx.x) * (kScatterBlock / 32) + (threadIdx.x >> 5)) * W;
-  if (w0 >= m.nwords) return;
+  grid_release();
+  if (w0 >= m.nwords) {
+    grid_wait();
+    return;
+  }
   const int K = KC ? KC : K_in;
   NodeWord w[W];
 #pragma unroll
@@ -53,6 +57,7 @@ __global__ void __launch_bounds__(kScatterBlock) ogs_scatter_kernel(const DevNod
     if (r[j] >= 0) r[j] = checked_id(r[j], nrows, err);
     if (NONLY && !((m.nmem[w0 + j] >> lane) & 1u)) r[j] = -1;
   }
+  grid_wait();
   for (int p0 = 0; p0 < K; p0 += B) {
     T x[W][B];
     int32_t row[W][B];
@@ -92,10 +97,8 @@ inline cudaError_t launch_scatter_as(const DevMaps& m, const FieldArgs& f, cudaS
   const unsigned grid = static_cast<unsigned>((m.nodes.nwords + per_block - 1) / per_block);
   // division by K as a multiply-high, exact while (32 K) K < 2^32
   const uint32_t kmagic = f.K < 11585 ? 0xFFFFFFFFu / static_cast<uint32_t>(f.K) + 1u : 0u;
-  ogs_scatter_kernel<T, KC, NONLY><<<grid, kScatterBlock, 0, s>>>(m.nodes, static_cast<T*>(f.v),
-                                                                  static_cast<const T*>(f.gv), f.K, kmagic,
-                                                                  m.b[1].nrows, m.b[1].err);
-  return cudaGetLastError();
+  return launch_overlapped(ogs_scatter_kernel<T, KC, NONLY>, dim3(grid), kScatterBlock, 0, s, f.overlap, m.nodes,
+                           static_cast<T*>(f.v), static_cast<const T*>(f.gv), f.K, kmagic, m.b[1].nrows, m.b[1].err);
 }
 
 template <typename T, bool NONLY>

@@ -171,6 +171,8 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_warp_kernel(const D
   const int64_t nw = m.nwtiles;
   const int64_t nitems = nw * K;
   int64_t i = static_cast<int64_t>(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5);
+  grid_release();
+  if (!PLAIN || i >= nitems) grid_wait();
   if (i >= nitems) return;
   const bool use_mask = !PLAIN && (pat.gather_n || pat.scatter_n) && m.signed_maps;
   const bool gmask = !PLAIN && pat.gather_n != 0;
@@ -206,6 +208,7 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_warp_kernel(const D
   if (i + W < nitems) nxt = m.wtiles[tile_of(i + W)];
 
   T* gv = static_cast<T*>(f.gv);
+  if (PLAIN) grid_wait();  // (as in ogs_async.cuh)
   for (;;) {
     const int k0 = ccur;
     const T* src = (MODE == kModeScatter) ? nullptr : field_base<T>(f, k0);
@@ -261,7 +264,7 @@ template <typename T, int OP, int MODE, int KL, bool PLAIN>
 inline void launch_warp_kl(const DevMaps& m, const FieldArgs& f, Pattern pat, cudaStream_t s) {
   const int64_t nitems = static_cast<int64_t>(m.nwtiles) * (KL == kK1 ? 1 : f.K);
   const int grid = warp_grid<T, OP, MODE, KL, PLAIN>(nitems);
-  ogs_warp_kernel<T, OP, MODE, KL, PLAIN><<<grid, kBlock, 0, s>>>(m, f, pat);
+  launch_overlapped(ogs_warp_kernel<T, OP, MODE, KL, PLAIN>, grid, kBlock, 0, s, f.overlap, m, f, pat);
 }
 
 template <typename T, int OP, int MODE, bool PLAIN>
