@@ -68,8 +68,8 @@ __device__ __forceinline__ void cp_async_wait() {
 
 // `lane` picks the tile rows (rows lane, lane + 32, ...); entry e of the
 // thread lives at stage[e * 32 + slot], slot = the thread's own lane.
-template <typename T, int MODE, int D>
-__device__ __forceinline__ void async_issue_vals(const WarpState& s, const T* src, const T* gv, int64_t stride, int K,
+template <typename T, int MODE, int D, typename S>
+__device__ __forceinline__ void async_issue_vals(const WarpState& s, const T* src, const T* gv, S stride, int K,
                                                  int k, bool gmask, int lane, int slot, T* stage) {
   constexpr int RPT = warp_rows_per_lane(D);
 #pragma unroll
@@ -81,7 +81,7 @@ __device__ __forceinline__ void async_issue_vals(const WarpState& s, const T* sr
 #pragma unroll
         for (int q = 0; q < D; ++q)
           if (!gmask || ((s.emask >> (j * D + q)) & 1u))
-            cp_async_elem(stage + (j * D + q) * 32 + slot, src + static_cast<int64_t>(s.I[j * D + q]) * stride);
+            cp_async_elem(stage + (j * D + q) * 32 + slot, value_at(src, s.I[j * D + q], stride));
       }
     }
   }
@@ -141,10 +141,13 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_async_kernel(const 
   // slower: 83 vs 62 us for k = 3 on 3.5 M permuted nodes.)  Items are
   // followed as (tile, part) pairs, advanced by W without division.
   const int64_t i0 = wid;
-  // The plain builds read descriptors and column ids before they wait for the
-  // work ahead (grid_wait); in the others the wait among them costs spills.
+  // Plain k = 1 reads descriptors and column ids before it waits for the work
+  // ahead (grid_wait).  With components the wait in the middle costs more
+  // registers than it hides: 32x32x16 p=5 permuted k=3 fp32 27.3 us a call
+  // against 26.4 with the wait up here, Gather 23.0 against 18.6.
   grid_release();
-  if (!PLAIN || i0 >= nitems) grid_wait();
+  constexpr bool kLate = PLAIN && KL == kK1;
+  if (!kLate || i0 >= nitems) grid_wait();
   if (i0 >= nitems) return;
   int64_t i = i0;
   const int64_t step = W, iend = nitems;
@@ -160,7 +163,7 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_async_kernel(const 
   const bool gmask = !PLAIN && pat.gather_n != 0;
   const int smode = PLAIN ? 0 : pat.scatter_n;
   const bool gslib = !PLAIN && pat.gslib != 0;
-  const int64_t stride = KL == kKInterleaved ? K : 1;
+  const ByteStride stride{(KL == kKInterleaved ? static_cast<uint32_t>(K) : 1u) * static_cast<uint32_t>(sizeof(T))};
   // the item W after (t, c)
   auto advance = [&](int t, int c, int& tn, int& cn) {
     if (KL == kK1) {
@@ -223,7 +226,7 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_async_kernel(const 
     OGS_DEGREE_SWITCH(nxt.bucket, OGS_A_LOAD_NXT)
 #undef OGS_A_LOAD_NXT
   }
-  if (PLAIN) grid_wait();  // the first access to the field follows
+  if (kLate) grid_wait();  // the first access to the field follows
   {
     const T* src = (MODE == kModeScatter) ? nullptr : field_base<T>(f, kcur);
 #define OGS_A_ISSUE0(D) async_issue_vals<T, MODE, D>(scur, src, gv, stride, K, kcur, gmask, rcur, lane, ring)

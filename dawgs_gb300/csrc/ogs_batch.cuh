@@ -167,7 +167,7 @@ __global__ void __launch_bounds__(BLOCK, OCC * 256 / BLOCK)
     const int smode = PLAIN ? 0 : (cur.flags >> 5) & 1;
     T* base = static_cast<T*>(cur.v) + k;
     T V[kWarpSlots];
-#define OGS_B_VALS(D) warp_load_vals<T, kModeGS, D>(scur, base, nullptr, K, K, k, gmask, rl, V)
+#define OGS_B_VALS(D) warp_load_vals<T, kModeGS, D>(scur, base, nullptr, static_cast<int64_t>(K), K, k, gmask, rl, V)
     OGS_DEGREE_SWITCH(d, OGS_B_VALS)
 #undef OGS_B_VALS
     WarpState snxt;
@@ -312,7 +312,7 @@ __global__ void __launch_bounds__(kBlock, OCC)
     const T* src = static_cast<const T*>(be.v) + cur.k;
     const bool gmask = !PLAIN && be.gather_n != 0;
 #define OGS_BA_ISSUE0(D) \
-  async_issue_vals<T, kModeGS, D>(scur, src, nullptr, be.K, be.K, cur.k, gmask, pos_lane(cur), lane, ring)
+  async_issue_vals<T, kModeGS, D>(scur, src, nullptr, static_cast<int64_t>(be.K), be.K, cur.k, gmask, pos_lane(cur), lane, ring)
     OGS_DEGREE_SWITCH(pos_deg(cur), OGS_BA_ISSUE0)
 #undef OGS_BA_ISSUE0
   }
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(kBlock, OCC)
       const bool gmask1 = !PLAIN && be.gather_n != 0;
       T* st1 = ring + nstage * (kWarpSlots * 32);
 #define OGS_BA_ISSUE1(D) \
-  async_issue_vals<T, kModeGS, D>(snxt, src1, nullptr, be.K, be.K, nxt.k, gmask1, pos_lane(nxt), lane, st1)
+  async_issue_vals<T, kModeGS, D>(snxt, src1, nullptr, static_cast<int64_t>(be.K), be.K, nxt.k, gmask1, pos_lane(nxt), lane, st1)
       OGS_DEGREE_SWITCH(pos_deg(nxt), OGS_BA_ISSUE1)
 #undef OGS_BA_ISSUE1
     }

@@ -159,6 +159,22 @@ __device__ __forceinline__ T* field_base(const FieldArgs& f, int k) {
   return f.is_many ? static_cast<T*>(f.many[k]) : static_cast<T*>(f.v) + k;
 }
 
+// Value `i` of a component, values a stride apart: in bytes below 2^32, a
+// product and sum in one instruction instead of three (21x18x20 p=7 masked
+// Trans k=2 30.9 -> 26.9 us a call, 24^3 p=3 k=8 21.2 -> 18.6), or in values.
+struct ByteStride {
+  uint32_t bytes;
+};
+template <typename T>
+__device__ __forceinline__ T* value_at(T* base, int32_t i, ByteStride s) {
+  using C = typename std::conditional<std::is_const<T>::value, const char, char>::type;
+  return reinterpret_cast<T*>(reinterpret_cast<C*>(base) + static_cast<uint64_t>(static_cast<uint32_t>(i)) * s.bytes);
+}
+template <typename T>
+__device__ __forceinline__ T* value_at(T* base, int32_t i, int64_t stride) {
+  return base + static_cast<int64_t>(i) * stride;
+}
+
 // Rows of exact degree D.
 template <typename T, int OP, int MODE, bool K1, int D>
 __device__ __forceinline__ void run_fixed(const DevBucket& b, const Tile& t, const FieldArgs& f,

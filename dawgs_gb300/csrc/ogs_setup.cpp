@@ -517,6 +517,7 @@ void set_id_bounds(const ogs_handle_s* h, DevMaps& m, unsigned int* err) {
 DevMaps general_maps(const DevMaps& m) {
   DevMaps g = m;
   g.nwtiles = 0;
+  g.tiles = g.gtiles;
   g.ntiles = g.ngtiles;
   return g;
 }

@@ -85,8 +85,8 @@ __device__ __forceinline__ void warp_load_state(const DevBucket& b, const Tile& 
   }
 }
 
-template <typename T, int MODE, int D>
-__device__ __forceinline__ void warp_load_vals(const WarpState& s, const T* src, const T* gv, int64_t stride,
+template <typename T, int MODE, int D, typename S>
+__device__ __forceinline__ void warp_load_vals(const WarpState& s, const T* src, const T* gv, S stride,
                                                int K, int k, bool gmask, int lane, T (&V)[kWarpSlots]) {
   constexpr int RPT = warp_rows_per_lane(D);
 #pragma unroll
@@ -97,7 +97,7 @@ __device__ __forceinline__ void warp_load_vals(const WarpState& s, const T* src,
       } else {
 #pragma unroll
         for (int q = 0; q < D; ++q)
-          if (!gmask || ((s.emask >> (j * D + q)) & 1u)) V[j * D + q] = src[static_cast<int64_t>(s.I[j * D + q]) * stride];
+          if (!gmask || ((s.emask >> (j * D + q)) & 1u)) V[j * D + q] = *value_at(src, s.I[j * D + q], stride);
       }
     }
   }
@@ -106,8 +106,8 @@ __device__ __forceinline__ void warp_load_vals(const WarpState& s, const T* src,
 // smode: 0 write every member, 1 only N members, 2 N members or, in a row
 // without any, member 0 (gslib transpose 1).  gslib: fold from the first
 // member taking part instead of from the identity (gs_local.c:58-72).
-template <typename T, int OP, int MODE, int D>
-__device__ __forceinline__ void warp_fold_store(const WarpState& s, T* dst, T* gv, int64_t stride, int K, int k,
+template <typename T, int OP, int MODE, int D, typename S>
+__device__ __forceinline__ void warp_fold_store(const WarpState& s, T* dst, T* gv, S stride, int K, int k,
                                                 bool gmask, int smode, bool gslib, int lane,
                                                 const T (&V)[kWarpSlots]) {
   constexpr int RPT = warp_rows_per_lane(D);
@@ -142,7 +142,7 @@ __device__ __forceinline__ void warp_fold_store(const WarpState& s, T* dst, T* g
           if (smode == 2 && !(row_n ? in_n : q == 0)) continue;
           // a member that took part in the fold still holds its value in V
           if (OGS_SILENT_STORE && MODE == kModeGS && (!gmask || in_n) && same_bits(a, V[j * D + q])) continue;
-          dst[static_cast<int64_t>(s.I[j * D + q]) * stride] = a;
+          *value_at(dst, s.I[j * D + q], stride) = a;
         }
       }
     }
@@ -172,13 +172,14 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_warp_kernel(const D
   const int64_t nitems = nw * K;
   int64_t i = static_cast<int64_t>(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5);
   grid_release();
-  if (!PLAIN || i >= nitems) grid_wait();
+  constexpr bool kLate = PLAIN && KL == kK1;
+  if (!kLate || i >= nitems) grid_wait();
   if (i >= nitems) return;
   const bool use_mask = !PLAIN && (pat.gather_n || pat.scatter_n) && m.signed_maps;
   const bool gmask = !PLAIN && pat.gather_n != 0;
   const int smode = PLAIN ? 0 : pat.scatter_n;
   const bool gslib = !PLAIN && pat.gslib != 0;
-  const int64_t stride = KL == kKInterleaved ? K : 1;
+  const ByteStride stride{(KL == kKInterleaved ? static_cast<uint32_t>(K) : 1u) * static_cast<uint32_t>(sizeof(T))};
   auto tile_of = [&](int64_t item) {
     return static_cast<int>(KL == kKMany ? item % nw : (KL == kKInterleaved ? item / K : item));
   };
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_warp_kernel(const D
   if (i + W < nitems) nxt = m.wtiles[tile_of(i + W)];
 
   T* gv = static_cast<T*>(f.gv);
-  if (PLAIN) grid_wait();  // (as in ogs_async.cuh)
+  if (kLate) grid_wait();  // (as in ogs_async.cuh)
   for (;;) {
     const int k0 = ccur;
     const T* src = (MODE == kModeScatter) ? nullptr : field_base<T>(f, k0);
