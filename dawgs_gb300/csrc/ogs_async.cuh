@@ -105,6 +105,86 @@ __device__ __forceinline__ void async_read_vals(const WarpState& s, bool gmask, 
   }
 }
 
+// ---- lone tiles: 256 consecutive nodes, of which a byte per lane says which
+// are their row's only member.  Their values come in 16-byte vectors, without
+// column ids, and go back only if the fold from the identity changes their
+// bits.  The degree-1 tiles of a mesh of high degree cost 4 of every 12 bytes a
+// node moved and gathers of eight lines each: 24^3 p=15 fp64 185.7 -> 158.0 us.
+
+// Whether identity (+) x has x's bits for every x: integer Add and Min, and
+// Mul of every type (the fold starts from the member).  Lone tiles then have
+// nothing to do.
+template <typename T, int OP>
+OGS_HD constexpr bool lone_is_noop() {
+  return OP == OGS_MUL || (std::is_integral<T>::value && (OP == OGS_ADD || OP == OGS_MIN));
+}
+
+// Whether identity (+) x may differ from x: -0 under Add, infinities and NaN
+// under Max and Min, by their bits (a compare of 8-byte floats costs a warp 16
+// cycles of their pipe; 20^3 p=11 fp64 Max 45 us a call with it).
+template <typename T, int OP>
+__device__ __forceinline__ bool lone_suspect(const T x) {
+  if constexpr (std::is_floating_point<T>::value) {
+    using U = typename std::conditional<sizeof(T) == 8, unsigned long long, unsigned int>::type;
+    constexpr U sign = U(1) << (8 * sizeof(T) - 1);
+    constexpr U expo = sizeof(T) == 8 ? U(0x7FF0000000000000ull) : U(0x7F800000u);
+    U b;
+    memcpy(&b, &x, sizeof(T));
+    return OP == OGS_ADD ? b == sign : (b & expo) == expo;
+  } else {
+    return x < -type_max<T>();  // Max starts there
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ void lone_load_state(const DevMaps& m, const Tile& t, int lane, WarpState& s) {
+  s.I[0] = t.begin;
+  s.emask = __ldg((sizeof(T) == 8 ? m.lmask8 : m.lmask4) + static_cast<int64_t>(t.count) * 32 + lane);
+}
+
+template <typename T, int OP>
+__device__ __forceinline__ void lone_issue(const WarpState& s, const T* src, int N, int lane, T* stage) {
+  if (lone_is_noop<T, OP>()) return;
+  constexpr int VEC = 16 / sizeof(T);
+#pragma unroll
+  for (int j = 0; j < 8 / VEC; ++j) {
+    const int at = (j * 32 + lane) * VEC;
+    if (!((s.emask >> (j * VEC)) & ((1u << VEC) - 1u))) continue;
+    if (s.I[0] + at + VEC <= N) {
+      const unsigned to = static_cast<unsigned>(__cvta_generic_to_shared(stage + at));
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(to), "l"(src + s.I[0] + at) : "memory");
+    } else {  // the field's last vector
+#pragma unroll
+      for (int i = 0; i < VEC; ++i)
+        if (s.I[0] + at + i < N) cp_async_elem(stage + at + i, src + s.I[0] + at + i);
+    }
+  }
+}
+
+template <typename T, int OP>
+__device__ __forceinline__ void lone_fold_store(const WarpState& s, T* dst, int lane, const T* stage) {
+  if (lone_is_noop<T, OP>()) return;
+  constexpr int VEC = 16 / sizeof(T);
+#pragma unroll
+  for (int j = 0; j < 8 / VEC; ++j) {
+    const int at = (j * 32 + lane) * VEC;
+    alignas(16) T x[VEC];
+    *reinterpret_cast<uint4*>(x) = *reinterpret_cast<const uint4*>(stage + at);
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+      if (!lone_suspect<T, OP>(x[i]) || !((s.emask >> (j * VEC + i)) & 1u)) continue;
+      T a;
+      if constexpr (OP == OGS_ADD || OP == OGS_MUL) {
+        a = fold_from_first<T, OP, 1>(x, i);
+      } else {
+        a = op_init<T, OP>();
+        op_apply<T, OP>(a, x[i]);
+      }
+      if (!same_bits(a, x[i])) dst[s.I[0] + at + i] = a;
+    }
+  }
+}
+
 template <typename T>
 constexpr size_t async_smem_bytes() {
   return static_cast<size_t>(kBlock / 32) * kAsyncStages * kWarpSlots * 32 * sizeof(T);
@@ -113,7 +193,9 @@ constexpr size_t async_smem_bytes() {
 // PLAIN: every member takes part and receives the result (Pattern all zero:
 // GatherScatter Sym, Gather/Scatter through the T map) -- the member-mask,
 // store-mode and gslib branches drop out at compile time.
-template <typename T, int OP, int MODE, int KL, bool PLAIN>
+// LONE: the tiles are DevMaps::ltiles (plain GatherScatter, k = 1 or separate
+// arrays on 16-byte boundaries).
+template <typename T, int OP, int MODE, int KL, bool PLAIN, bool LONE>
 __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_async_kernel(const DevMaps m, const FieldArgs f,
                                                                           const Pattern pat_in) {
   const Pattern pat = PLAIN ? Pattern{0, 0, 0, 0} : pat_in;
@@ -217,20 +299,23 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_async_kernel(const 
   WarpState scur, snxt;
 #define OGS_A_LOAD(D, TILE, TI, RL, S) warp_load_state<MODE, D>(m.b[D], TILE, m.wemask, TI, use_mask, pat, RL, S)
 #define OGS_A_LOAD_CUR(D) OGS_A_LOAD(D, cur, tcur, rcur, scur)
-  OGS_DEGREE_SWITCH(cur.bucket, OGS_A_LOAD_CUR)
+  if (LONE && cur.bucket == kLoneBucket) lone_load_state<T>(m, cur, lane, scur);
+  else OGS_DEGREE_SWITCH(cur.bucket, OGS_A_LOAD_CUR)
 #undef OGS_A_LOAD_CUR
   if (has1) {
     int rnxt, knxt;
     unit(cnxt, rnxt, knxt);
 #define OGS_A_LOAD_NXT(D) OGS_A_LOAD(D, nxt, tnxt, rnxt, snxt)
-    OGS_DEGREE_SWITCH(nxt.bucket, OGS_A_LOAD_NXT)
+    if (LONE && nxt.bucket == kLoneBucket) lone_load_state<T>(m, nxt, lane, snxt);
+    else OGS_DEGREE_SWITCH(nxt.bucket, OGS_A_LOAD_NXT)
 #undef OGS_A_LOAD_NXT
   }
   if (kLate) grid_wait();  // the first access to the field follows
   {
     const T* src = (MODE == kModeScatter) ? nullptr : field_base<T>(f, kcur);
 #define OGS_A_ISSUE0(D) async_issue_vals<T, MODE, D>(scur, src, gv, stride, K, kcur, gmask, rcur, lane, ring)
-    OGS_DEGREE_SWITCH(cur.bucket, OGS_A_ISSUE0)
+    if (LONE && cur.bucket == kLoneBucket) lone_issue<T, OP>(scur, src, m.b[1].nnodes, lane, ring);
+    else OGS_DEGREE_SWITCH(cur.bucket, OGS_A_ISSUE0)
 #undef OGS_A_ISSUE0
   }
   cp_async_commit();
@@ -246,7 +331,8 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_async_kernel(const 
       const T* src1 = (MODE == kModeScatter) ? nullptr : field_base<T>(f, knxt);
       T* st1 = ring + nstage * (kWarpSlots * 32);
 #define OGS_A_ISSUE1(D) async_issue_vals<T, MODE, D>(snxt, src1, gv, stride, K, knxt, gmask, rnxt, lane, st1)
-      OGS_DEGREE_SWITCH(nxt.bucket, OGS_A_ISSUE1)
+      if (LONE && nxt.bucket == kLoneBucket) lone_issue<T, OP>(snxt, src1, m.b[1].nnodes, lane, st1);
+      else OGS_DEGREE_SWITCH(nxt.bucket, OGS_A_ISSUE1)
 #undef OGS_A_ISSUE1
     }
     cp_async_commit();
@@ -257,7 +343,8 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_async_kernel(const 
       int rnn, knn;
       unit(cnn, rnn, knn);
 #define OGS_A_LOAD_NN(D) OGS_A_LOAD(D, nn, tnn, rnn, snn)
-      OGS_DEGREE_SWITCH(nn.bucket, OGS_A_LOAD_NN)
+      if (LONE && nn.bucket == kLoneBucket) lone_load_state<T>(m, nn, lane, snn);
+      else OGS_DEGREE_SWITCH(nn.bucket, OGS_A_LOAD_NN)
 #undef OGS_A_LOAD_NN
       if (i + 3 * step < iend) {
         advance(tnn, cnn, tn3, cn3);
@@ -275,7 +362,8 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_async_kernel(const 
     async_read_vals<T, MODE, D>(scur, gmask, rcur, lane, st0, V);                                  \
     warp_fold_store<T, OP, MODE, D>(scur, dst, gv, stride, K, kcur, gmask, smode, gslib, rcur, V); \
   } while (0)
-      OGS_DEGREE_SWITCH(cur.bucket, OGS_A_FOLD)
+      if (LONE && cur.bucket == kLoneBucket) lone_fold_store<T, OP>(scur, dst, lane, st0);
+      else OGS_DEGREE_SWITCH(cur.bucket, OGS_A_FOLD)
 #undef OGS_A_FOLD
     }
     if (!more1) break;
@@ -297,7 +385,7 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_async_kernel(const 
 #undef OGS_A_LOAD
 }
 
-template <typename T, int OP, int MODE, int KL, bool PLAIN>
+template <typename T, int OP, int MODE, int KL, bool PLAIN, bool LONE>
 inline int async_grid(int64_t nitems) {
   static DeviceCache cache;
   int dev = 0;
@@ -306,9 +394,9 @@ inline int async_grid(int64_t nitems) {
     int bps = 0, sms = 0;
     // above 48 KB (more entries per lane) the dynamic shared memory must be opted into
     if (async_smem_bytes<T>() > 48 * 1024)
-      cudaFuncSetAttribute(ogs_async_kernel<T, OP, MODE, KL, PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+      cudaFuncSetAttribute(ogs_async_kernel<T, OP, MODE, KL, PLAIN, LONE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            static_cast<int>(async_smem_bytes<T>()));
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, ogs_async_kernel<T, OP, MODE, KL, PLAIN>, kBlock,
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, ogs_async_kernel<T, OP, MODE, KL, PLAIN, LONE>, kBlock,
                                                   async_smem_bytes<T>());
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
 #if OGS_ASYNC_CTAS > 0
@@ -320,17 +408,29 @@ inline int async_grid(int64_t nitems) {
   return static_cast<int>(need < cached ? need : cached);
 }
 
+template <typename T, int OP, int MODE, int KL, bool PLAIN, bool LONE>
+inline void launch_async_as(const DevMaps& m, const FieldArgs& f, Pattern pat, cudaStream_t s) {
+  const int grid = async_grid<T, OP, MODE, KL, PLAIN, LONE>(static_cast<int64_t>(m.nwtiles) * (KL == kK1 ? 1 : f.K));
+  launch_overlapped(ogs_async_kernel<T, OP, MODE, KL, PLAIN, LONE>, dim3(grid), kBlock, async_smem_bytes<T>(), s,
+                    f.overlap, m, f, pat);
+}
+
 template <typename T, int OP, int MODE, int KL>
 inline void launch_async_kl(const DevMaps& m, const FieldArgs& f, Pattern pat, cudaStream_t s) {
-  const int64_t nitems = static_cast<int64_t>(m.nwtiles) * (KL == kK1 ? 1 : f.K);
   const bool plain = !pat.gather_n && !pat.scatter_n && !pat.limit_n && !pat.gslib;
-  if (plain) {
-    const int grid = async_grid<T, OP, MODE, KL, true>(nitems);
-    launch_overlapped(ogs_async_kernel<T, OP, MODE, KL, true>, grid, kBlock, async_smem_bytes<T>(), s, f.overlap, m, f, pat);
-  } else {
-    const int grid = async_grid<T, OP, MODE, KL, false>(nitems);
-    launch_overlapped(ogs_async_kernel<T, OP, MODE, KL, false>, grid, kBlock, async_smem_bytes<T>(), s, f.overlap, m, f, pat);
+  if constexpr (MODE == kModeGS && KL != kKInterleaved) {
+    bool lone = plain && m.nltiles > 0;
+    for (int k = 0; lone && k < (KL == kKMany ? f.K : 1); ++k)
+      lone = (reinterpret_cast<uintptr_t>(KL == kKMany ? f.many[k] : f.v) & 15) == 0;
+    if (lone) {
+      DevMaps l = m;
+      l.wtiles = m.ltiles;
+      l.nwtiles = m.nltiles;
+      return launch_async_as<T, OP, MODE, KL, true, true>(l, f, pat, s);
+    }
   }
+  if (plain) launch_async_as<T, OP, MODE, KL, true, false>(m, f, pat, s);
+  else launch_async_as<T, OP, MODE, KL, false, false>(m, f, pat, s);
 }
 
 // Exact-degree tiles on the async pipeline, general rows in a launch of their own.

@@ -349,6 +349,29 @@ __global__ void k_wemask(const Tile* __restrict__ wt, int64_t nw, BucketPtrs B, 
   wemask[x] = static_cast<uint8_t>(bits);
 }
 
+// Lone nodes as bits, and the lone tiles' masks from them.
+__global__ void k_lone_bits(const int32_t* __restrict__ cols, int64_t n, uint32_t* __restrict__ bits) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * kT + threadIdx.x;
+  if (i < n) atomicOr(&bits[cols[i] >> 5], 1u << (cols[i] & 31));
+}
+
+__global__ void k_lone_masks(const uint32_t* __restrict__ bits, int64_t n, uint8_t* __restrict__ m8,
+                             uint8_t* __restrict__ m4) {
+  const int64_t x = static_cast<int64_t>(blockIdx.x) * kT + threadIdx.x;
+  if (x >= n) return;
+  const int64_t n0 = (x >> 5) * kLoneNodes;
+  const int lane = static_cast<int>(x & 31);
+  uint32_t a = 0, b = 0;
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const int64_t p = n0 + lone_node(lane, q, 2), r = n0 + lone_node(lane, q, 4);
+    a |= ((bits[p >> 5] >> (p & 31)) & 1u) << q;
+    b |= ((bits[r >> 5] >> (r & 31)) & 1u) << q;
+  }
+  m8[x] = static_cast<uint8_t>(a);
+  m4[x] = static_cast<uint8_t>(b);
+}
+
 // Ids of the wide tiles (DevMaps::wide), a warp per tile.
 __global__ void k_wide_ids(const Tile* __restrict__ wide, int64_t nwide, const int32_t* __restrict__ startsT,
                            const int32_t* __restrict__ colsT, const int32_t* __restrict__ startsN,
@@ -600,6 +623,16 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
   const size_t o_wtiles = add(L.wtiles.size() * sizeof(Tile));
   const size_t o_wemask = add(sgn ? L.wtiles.size() * 32 : 0);
   const int64_t wide_units = wide_layout(g_startsT.data(), ng, L.wide);
+  // lone tiles: their number now, the tiles when the tiles' lowest nodes are known
+  const bool lone = wants_lone(h, L.n[1]);
+  int64_t nlt = 0;
+  if (lone) {
+    nlt = lone_tiles(h->N);
+    for (const Tile& w : L.wtiles) nlt += w.bucket != 1;
+  }
+  const int64_t nlm = lone ? lone_tiles(h->N) * 32 : 0;
+  const size_t o_lt = add(static_cast<size_t>(nlt) * sizeof(Tile));
+  const size_t o_lm8 = add(static_cast<size_t>(nlm)), o_lm4 = add(static_cast<size_t>(nlm));
   const size_t o_wide = add(L.wide.size() * sizeof(Tile));
   const size_t o_wids = add(static_cast<size_t>(wide_units) * 32 * 4);
   const bool words = wants_node_words(h);
@@ -671,6 +704,15 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
   if (nw + ngt)
     k_tile_bounds<<<nblocks((nw + ngt) * 32), kT, 0, st>>>(d_wt, nw, B, d_gt, ngt, g_sT, g_cT, d_lo, d_hi);
   if (sgn && nw) k_wemask<<<nblocks(nw * 32), kT, 0, st>>>(d_wt, nw, B, reinterpret_cast<uint8_t*>(base + o_wemask));
+  if (lone) {
+    uint32_t* bits = nullptr;
+    const int64_t nb = lone_tiles(h->N) * (kLoneNodes / 32);
+    if ((e = sc.get(&bits, nb))) return release(e, "allocation");
+    if ((e = cudaMemsetAsync(bits, 0, static_cast<size_t>(nb) * 4, st))) return release(e, "memset");
+    k_lone_bits<<<nblocks(L.n[1]), kT, 0, st>>>(B.cols[1], L.n[1], bits);
+    k_lone_masks<<<nblocks(nlm), kT, 0, st>>>(bits, nlm, reinterpret_cast<uint8_t*>(base + o_lm8),
+                                              reinterpret_cast<uint8_t*>(base + o_lm4));
+  }
   NodeWord* d_words = reinterpret_cast<NodeWord*>(base + o_words);
   if (words) {
     int32_t *others = nullptr, *other0 = nullptr;
@@ -696,6 +738,12 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
   L.glo.assign(lo.begin() + nw, lo.end());
   L.ghi.assign(hi.begin() + nw, hi.end());
   build_phases(h, OGS_HOST_PHASES);
+  lone_layout(h);
+  if (lone) {
+    e = cudaMemcpyAsync(base + o_lt, L.ltiles.data(), L.ltiles.size() * sizeof(Tile), cudaMemcpyHostToDevice, st);
+    if (!e) e = cudaStreamSynchronize(st);
+    if (e) return release(e, "lone tiles");
+  }
 
   h->device = dev;
   h->arena = base;
@@ -725,6 +773,10 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
   m.nwtiles = static_cast<int32_t>(nw);
   m.wemask = reinterpret_cast<const uint8_t*>(base + o_wemask);
   m.wrecs = reinterpret_cast<const WarpRec*>(base + o_wrecs);
+  m.ltiles = reinterpret_cast<const Tile*>(base + o_lt);
+  m.lmask8 = reinterpret_cast<const uint8_t*>(base + o_lm8);
+  m.lmask4 = reinterpret_cast<const uint8_t*>(base + o_lm4);
+  m.nltiles = static_cast<int32_t>(nlt);
   m.wide = d_wide;
   m.wide_ids = d_wids;
   m.nwide = static_cast<int32_t>(nwide);

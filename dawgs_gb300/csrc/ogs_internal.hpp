@@ -186,6 +186,15 @@ constexpr int kNodeWordPad = 16;
 inline int64_t node_words(int64_t N) { return (N + 31) / 32; }
 inline int64_t node_words_padded(int64_t N) { return (node_words(N) + kNodeWordPad - 1) / kNodeWordPad * kNodeWordPad; }
 
+// Lone nodes (their row's only member) of kLoneNodes consecutive nodes, as a
+// tile of the exact-degree rows' launch (ogs_async.cuh): bucket kLoneBucket,
+// begin the first node, count the tile's row of the masks.
+constexpr int kLoneNodes = 256;
+constexpr int kLoneBucket = kDmax + 1;
+// Bit q of lane l's byte stands for node ((q / v) * 32 + l) * v + q % v of the
+// tile, v = 2 or 4 values of 8 or 4 bytes in a 16-byte vector.
+OGS_HD inline int lone_node(int l, int q, int v) { return ((q / v) * 32 + l) * v + q % v; }
+
 // Member of a wide tile's row: node | N member << 31, or none.
 constexpr uint32_t kNoWideId = 0xFFFFFFFFu;
 constexpr int kWideRows = 32;  // rows of a wide tile
@@ -209,6 +218,12 @@ struct DevMaps {
   const Tile* wide;
   const uint32_t* wide_ids;
   int32_t nwide;           // 0: the general rows run as CTA tiles
+  // The warp tiles of degree 2 and up with lone tiles in place of the degree-1
+  // ones, in node order, for handles that are mostly lone nodes (wants_lone).
+  const Tile* ltiles;
+  const uint8_t* lmask8;   // [lone tiles][32] for 8-byte values
+  const uint8_t* lmask4;   // ... for 4-byte values
+  int32_t nltiles;         // 0: the handle has none
 };
 
 // Which members take part, per ogsOperator.cpp:60-97, 206-238, 311-360.
@@ -264,6 +279,8 @@ struct HostLayout {
   std::vector<NodeWord> nwords;  // host path only: see DevNodes
   std::vector<uint32_t> nmem;
   std::vector<int32_t> orow;
+  std::vector<Tile> ltiles;        // see DevMaps
+  std::vector<uint8_t> lmask8, lmask4;  // host path only
   std::vector<Tile> wide;          // see DevMaps
   std::vector<uint32_t> wide_ids;  // host path only
   std::vector<Phase> phases;
@@ -338,6 +355,18 @@ inline bool wants_node_words(const ogs_handle_s* h) {
 // they take.  None where rows of very different degree are neighbours and the
 // padding would outweigh the rows.
 int64_t wide_layout(const int32_t* starts, int64_t rows, std::vector<Tile>& wide);
+// Whether a handle gets lone tiles for its n1 rows of degree 1 (the rows being
+// numbered by first member): from 55 % of its nodes on.  Us a call without and
+// with them, boxes of 24^3: fp64 p=9 (51 %) 47.7 and 49.0, p=10 (55 %) 60.0 and
+// 60.2, p=11 (58 %) 76.4 and 75.4, p=15 (67 %) 185.7 and 158.0; fp32 p=11 60.2
+// and 56.5, p=7 (42 %) 17.5 and 19.1.
+inline bool wants_lone(const ogs_handle_s* h, int64_t n1) {
+  return !h->gslib && !h->from_maps && h->NlocalP == h->NlocalT && n1 * 20 >= h->N * 11;
+}
+// The lone tiles of N nodes; and HostLayout::ltiles (needs the warp tiles and the
+// lowest node of each).
+inline int64_t lone_tiles(int64_t N) { return (N + kLoneNodes - 1) / kLoneNodes; }
+void lone_layout(ogs_handle_s* h);
 // DevMaps restricted to the general rows.
 DevMaps general_maps(const DevMaps& m);
 // DevMaps restricted to the tiles of one phase.

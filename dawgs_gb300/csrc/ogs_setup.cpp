@@ -199,6 +199,24 @@ int64_t wide_layout(const int32_t* starts, int64_t rows, std::vector<Tile>& wide
   return units;
 }
 
+void lone_layout(ogs_handle_s* h) {
+  HostLayout& L = h->lay;
+  L.ltiles.clear();
+  if (!wants_lone(h, L.n[1])) return;
+  const int64_t n = lone_tiles(h->N);
+  int64_t c = 0;
+  auto lone_below = [&](int64_t node) {
+    for (; c < n && c * kLoneNodes <= node; ++c)
+      L.ltiles.push_back(Tile{kLoneBucket, static_cast<int32_t>(c * kLoneNodes), static_cast<int32_t>(c), 0});
+  };
+  for (size_t t = 0; t < L.wtiles.size(); ++t) {
+    if (L.wtiles[t].bucket == 1) continue;
+    lone_below(L.wlo[t]);
+    L.ltiles.push_back(L.wtiles[t]);
+  }
+  lone_below(h->N);
+}
+
 void build_layout(ogs_handle_s* h) {
   TraceRange trace("ogs_setup: layout on the host");
   HostLayout& L = h->lay;
@@ -384,6 +402,20 @@ void build_layout(ogs_handle_s* h) {
       L.ghi[t] = std::max<int64_t>(L.ghi[t], L.g_colsT[q]);
     }
   }
+  lone_layout(h);
+  L.lmask8.assign(L.ltiles.empty() ? 0 : lone_tiles(h->N) * 32, 0);
+  L.lmask4.assign(L.lmask8.size(), 0);
+  if (!L.ltiles.empty()) {
+    std::vector<uint8_t> lone(static_cast<size_t>(lone_tiles(h->N)) * kLoneNodes, 0);
+    for (int32_t i = 0; i < L.n[1]; ++i) lone[L.cols[1][i]] = 1;
+    for (size_t x = 0; x < L.lmask8.size(); ++x) {
+      const uint8_t* at = lone.data() + x / 32 * kLoneNodes;
+      for (int q = 0; q < 8; ++q) {
+        L.lmask8[x] |= static_cast<uint8_t>(at[lone_node(x % 32, q, 2)] << q);
+        L.lmask4[x] |= static_cast<uint8_t>(at[lone_node(x % 32, q, 4)] << q);
+      }
+    }
+  }
   build_phases(h, OGS_HOST_PHASES);
 }
 
@@ -516,7 +548,7 @@ void set_id_bounds(const ogs_handle_s* h, DevMaps& m, unsigned int* err) {
 
 DevMaps general_maps(const DevMaps& m) {
   DevMaps g = m;
-  g.nwtiles = 0;
+  g.nwtiles = g.nltiles = 0;
   g.tiles = g.gtiles;
   g.ntiles = g.ngtiles;
   return g;
@@ -527,7 +559,7 @@ DevMaps general_maps(const DevMaps& m) {
 DevMaps phase_maps(const DevMaps& m, const Phase& p) {
   DevMaps r = m;
   r.nodes.nwords = 0;
-  r.nwide = 0;
+  r.nwide = r.nltiles = 0;
   r.wtiles = m.wtiles + p.w0;
   r.nwtiles = p.w1 - p.w0;
   if (m.wemask) r.wemask = m.wemask + static_cast<int64_t>(p.w0) * 32;
@@ -582,6 +614,9 @@ ogs_status upload_layout(ogs_handle_s* h) {
   const size_t o_gtiles = add(L.gtiles.data(), L.gtiles.size() * sizeof(Tile));
   const size_t o_wtiles = add(L.wtiles.data(), L.wtiles.size() * sizeof(Tile));
   const size_t o_wemask = add(L.wemask.data(), L.wemask.size());
+  const size_t o_lt = add(L.ltiles.data(), L.ltiles.size() * sizeof(Tile));
+  const size_t o_lm8 = add(L.lmask8.data(), L.lmask8.size());
+  const size_t o_lm4 = add(L.lmask4.data(), L.lmask4.size());
   const size_t o_wide = add(L.wide.data(), L.wide.size() * sizeof(Tile));
   const size_t o_wids = add(L.wide_ids.data(), L.wide_ids.size() * 4);
   const size_t o_words = add(L.nwords.data(), L.nwords.size() * sizeof(NodeWord));
@@ -649,6 +684,10 @@ ogs_status upload_layout(ogs_handle_s* h) {
   m.nwtiles = static_cast<int32_t>(L.wtiles.size());
   m.wemask = reinterpret_cast<const uint8_t*>(base + o_wemask);
   m.wrecs = reinterpret_cast<const WarpRec*>(base + o_wrecs);
+  m.ltiles = reinterpret_cast<const Tile*>(base + o_lt);
+  m.lmask8 = reinterpret_cast<const uint8_t*>(base + o_lm8);
+  m.lmask4 = reinterpret_cast<const uint8_t*>(base + o_lm4);
+  m.nltiles = static_cast<int32_t>(L.ltiles.size());
   m.wide = reinterpret_cast<const Tile*>(base + o_wide);
   m.wide_ids = reinterpret_cast<const uint32_t*>(base + o_wids);
   m.nwide = static_cast<int32_t>(L.wide.size());
