@@ -356,20 +356,22 @@ __global__ void k_lone_bits(const int32_t* __restrict__ cols, int64_t n, uint32_
 }
 
 __global__ void k_lone_masks(const uint32_t* __restrict__ bits, int64_t n, uint8_t* __restrict__ m8,
-                             uint8_t* __restrict__ m4) {
+                             uint8_t* __restrict__ m4, uint8_t* __restrict__ m1) {
   const int64_t x = static_cast<int64_t>(blockIdx.x) * kT + threadIdx.x;
   if (x >= n) return;
   const int64_t n0 = (x >> 5) * kLoneNodes;
   const int lane = static_cast<int>(x & 31);
-  uint32_t a = 0, b = 0;
+  uint32_t a = 0, b = 0, c = 0;
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
+    c |= ((bits[(n0 >> 5) + q] >> lane) & 1u) << q;  // lone_node(lane, q, 1)
     const int64_t p = n0 + lone_node(lane, q, 2), r = n0 + lone_node(lane, q, 4);
     a |= ((bits[p >> 5] >> (p & 31)) & 1u) << q;
     b |= ((bits[r >> 5] >> (r & 31)) & 1u) << q;
   }
   m8[x] = static_cast<uint8_t>(a);
   m4[x] = static_cast<uint8_t>(b);
+  if (m1) m1[x] = static_cast<uint8_t>(c);
 }
 
 // Ids of the wide tiles (DevMaps::wide), a warp per tile.
@@ -633,6 +635,7 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
   const int64_t nlm = lone ? lone_tiles(h->N) * 32 : 0;
   const size_t o_lt = add(static_cast<size_t>(nlt) * sizeof(Tile));
   const size_t o_lm8 = add(static_cast<size_t>(nlm)), o_lm4 = add(static_cast<size_t>(nlm));
+  const size_t o_lm1 = add(wants_node_words(h) ? static_cast<size_t>(nlm) : 0);
   const size_t o_wide = add(L.wide.size() * sizeof(Tile));
   const size_t o_wids = add(static_cast<size_t>(wide_units) * 32 * 4);
   const bool words = wants_node_words(h);
@@ -711,7 +714,8 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
     if ((e = cudaMemsetAsync(bits, 0, static_cast<size_t>(nb) * 4, st))) return release(e, "memset");
     k_lone_bits<<<nblocks(L.n[1]), kT, 0, st>>>(B.cols[1], L.n[1], bits);
     k_lone_masks<<<nblocks(nlm), kT, 0, st>>>(bits, nlm, reinterpret_cast<uint8_t*>(base + o_lm8),
-                                              reinterpret_cast<uint8_t*>(base + o_lm4));
+                                              reinterpret_cast<uint8_t*>(base + o_lm4),
+                                              words ? reinterpret_cast<uint8_t*>(base + o_lm1) : nullptr);
   }
   NodeWord* d_words = reinterpret_cast<NodeWord*>(base + o_words);
   if (words) {
@@ -776,6 +780,7 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
   m.ltiles = reinterpret_cast<const Tile*>(base + o_lt);
   m.lmask8 = reinterpret_cast<const uint8_t*>(base + o_lm8);
   m.lmask4 = reinterpret_cast<const uint8_t*>(base + o_lm4);
+  m.lmask1 = reinterpret_cast<const uint8_t*>(base + o_lm1);
   m.nltiles = static_cast<int32_t>(nlt);
   m.wide = d_wide;
   m.wide_ids = d_wids;

@@ -192,7 +192,7 @@ inline int64_t node_words_padded(int64_t N) { return (node_words(N) + kNodeWordP
 constexpr int kLoneNodes = 256;
 constexpr int kLoneBucket = kDmax + 1;
 // Bit q of lane l's byte stands for node ((q / v) * 32 + l) * v + q % v of the
-// tile, v = 2 or 4 values of 8 or 4 bytes in a 16-byte vector.
+// tile, v = 2 or 4 values of 8 or 4 bytes in a 16-byte vector, or 1.
 OGS_HD inline int lone_node(int l, int q, int v) { return ((q / v) * 32 + l) * v + q % v; }
 
 // Member of a wide tile's row: node | N member << 31, or none.
@@ -223,6 +223,7 @@ struct DevMaps {
   const Tile* ltiles;
   const uint8_t* lmask8;   // [lone tiles][32] for 8-byte values
   const uint8_t* lmask4;   // ... for 4-byte values
+  const uint8_t* lmask1;   // ... a node at a time (handles with node words)
   int32_t nltiles;         // 0: the handle has none
 };
 
@@ -280,7 +281,7 @@ struct HostLayout {
   std::vector<uint32_t> nmem;
   std::vector<int32_t> orow;
   std::vector<Tile> ltiles;        // see DevMaps
-  std::vector<uint8_t> lmask8, lmask4;  // host path only
+  std::vector<uint8_t> lmask8, lmask4, lmask1;  // host path only
   std::vector<Tile> wide;          // see DevMaps
   std::vector<uint32_t> wide_ids;  // host path only
   std::vector<Phase> phases;
@@ -359,7 +360,9 @@ int64_t wide_layout(const int32_t* starts, int64_t rows, std::vector<Tile>& wide
 // numbered by first member): from 55 % of its nodes on.  Us a call without and
 // with them, boxes of 24^3: fp64 p=9 (51 %) 47.7 and 49.0, p=10 (55 %) 60.0 and
 // 60.2, p=11 (58 %) 76.4 and 75.4, p=15 (67 %) 185.7 and 158.0; fp32 p=11 60.2
-// and 56.5, p=7 (42 %) 17.5 and 19.1.
+// and 56.5, p=7 (42 %) 17.5 and 19.1.  Gather fp64 p=7 25.1 and 24.6, p=9 46.6
+// and 44.5, p=11 77.8 and 72.2, p=15 189.4 and 162.3; fp32 p=7 13.3 and 14.8,
+// p=11 55.8 and 54.8.
 inline bool wants_lone(const ogs_handle_s* h, int64_t n1) {
   return !h->gslib && !h->from_maps && h->NlocalP == h->NlocalT && n1 * 20 >= h->N * 11;
 }

@@ -405,6 +405,7 @@ void build_layout(ogs_handle_s* h) {
   lone_layout(h);
   L.lmask8.assign(L.ltiles.empty() ? 0 : lone_tiles(h->N) * 32, 0);
   L.lmask4.assign(L.lmask8.size(), 0);
+  L.lmask1.assign(L.nwords.empty() ? 0 : L.lmask8.size(), 0);
   if (!L.ltiles.empty()) {
     std::vector<uint8_t> lone(static_cast<size_t>(lone_tiles(h->N)) * kLoneNodes, 0);
     for (int32_t i = 0; i < L.n[1]; ++i) lone[L.cols[1][i]] = 1;
@@ -413,6 +414,7 @@ void build_layout(ogs_handle_s* h) {
       for (int q = 0; q < 8; ++q) {
         L.lmask8[x] |= static_cast<uint8_t>(at[lone_node(x % 32, q, 2)] << q);
         L.lmask4[x] |= static_cast<uint8_t>(at[lone_node(x % 32, q, 4)] << q);
+        if (!L.lmask1.empty()) L.lmask1[x] |= static_cast<uint8_t>(at[lone_node(x % 32, q, 1)] << q);
       }
     }
   }
@@ -617,6 +619,7 @@ ogs_status upload_layout(ogs_handle_s* h) {
   const size_t o_lt = add(L.ltiles.data(), L.ltiles.size() * sizeof(Tile));
   const size_t o_lm8 = add(L.lmask8.data(), L.lmask8.size());
   const size_t o_lm4 = add(L.lmask4.data(), L.lmask4.size());
+  const size_t o_lm1 = add(L.lmask1.data(), L.lmask1.size());
   const size_t o_wide = add(L.wide.data(), L.wide.size() * sizeof(Tile));
   const size_t o_wids = add(L.wide_ids.data(), L.wide_ids.size() * 4);
   const size_t o_words = add(L.nwords.data(), L.nwords.size() * sizeof(NodeWord));
@@ -687,6 +690,7 @@ ogs_status upload_layout(ogs_handle_s* h) {
   m.ltiles = reinterpret_cast<const Tile*>(base + o_lt);
   m.lmask8 = reinterpret_cast<const uint8_t*>(base + o_lm8);
   m.lmask4 = reinterpret_cast<const uint8_t*>(base + o_lm4);
+  m.lmask1 = reinterpret_cast<const uint8_t*>(base + o_lm1);
   m.nltiles = static_cast<int32_t>(L.ltiles.size());
   m.wide = reinterpret_cast<const Tile*>(base + o_wide);
   m.wide_ids = reinterpret_cast<const uint32_t*>(base + o_wids);

@@ -161,7 +161,45 @@ __device__ __forceinline__ void warp_fold_store(const WarpState& s, T* dst, T* g
     default: CALL(8); break;            \
   }
 
-template <typename T, int OP, int MODE, int KL, bool PLAIN>
+// Lone tiles of a Gather (DevMaps::ltiles): lane l takes nodes l, l + 32, ... of
+// the tile, and a node's row follows from its word's first members.
+__device__ __forceinline__ void lone_rows(const DevMaps& m, const Tile& t, int lane, WarpState& s) {
+  s.I[0] = t.begin;
+  s.emask = __ldg(m.lmask1 + static_cast<int64_t>(t.count) * 32 + lane);
+  const NodeWord* w = m.nodes.words + (t.begin >> 5);
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const uint2 f = __ldg(reinterpret_cast<const uint2*>(w + q));
+    const int32_t row0 = __ldg(&w[q].row0);
+    s.R[q] = checked_id(row0 + __popc(f.x & ((1u << lane) - 1u)), m.b[1].nrows, m.b[1].err);
+  }
+}
+
+template <typename T>
+__device__ __forceinline__ void lone_load_vals(const WarpState& s, const T* src, int lane, T (&V)[kWarpSlots]) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    if ((s.emask >> q) & 1u) V[q] = src[s.I[0] + q * 32 + lane];
+}
+
+template <typename T, int OP>
+__device__ __forceinline__ void lone_gather(const WarpState& s, T* gv, const T (&V)[kWarpSlots]) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    if ((s.emask >> q) & 1u) {
+      T a;
+      if constexpr (OP == OGS_ADD || OP == OGS_MUL) {
+        a = fold_from_first<T, OP, 1>(V, q);
+      } else {
+        a = op_init<T, OP>();
+        op_apply<T, OP>(a, V[q]);
+      }
+      gv[s.R[q]] = a;
+    }
+}
+
+// LONE: the tiles are DevMaps::ltiles (plain Gather, k = 1).
+template <typename T, int OP, int MODE, int KL, bool PLAIN, bool LONE>
 __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_warp_kernel(const DevMaps m, const FieldArgs f,
                                                                          const Pattern pat_in) {
   const Pattern pat = PLAIN ? Pattern{0, 0, 0, 0} : pat_in;
@@ -203,7 +241,8 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_warp_kernel(const D
   int ccur;
   int rcur = row_lane(i, ccur);
 #define OGS_LOAD_CUR(D) warp_load_state<MODE, D>(m.b[D], cur, m.wemask, tcur, use_mask, pat, rcur, scur)
-  OGS_DEGREE_SWITCH(cur.bucket, OGS_LOAD_CUR)
+  if (LONE && cur.bucket == kLoneBucket) lone_rows(m, cur, lane, scur);
+  else OGS_DEGREE_SWITCH(cur.bucket, OGS_LOAD_CUR)
 #undef OGS_LOAD_CUR
   Tile nxt{};
   if (i + W < nitems) nxt = m.wtiles[tile_of(i + W)];
@@ -216,7 +255,8 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_warp_kernel(const D
     T* dst = (MODE == kModeGather) ? nullptr : field_base<T>(f, k0);
     T V[kWarpSlots];
 #define OGS_VALS(D) warp_load_vals<T, MODE, D>(scur, src, gv, stride, K, k0, gmask, rcur, V)
-    OGS_DEGREE_SWITCH(cur.bucket, OGS_VALS)
+    if (LONE && cur.bucket == kLoneBucket) lone_load_vals(scur, src, lane, V);
+    else OGS_DEGREE_SWITCH(cur.bucket, OGS_VALS)
 #undef OGS_VALS
     const bool more = i + W < nitems;
     WarpState snxt;
@@ -226,12 +266,14 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_warp_kernel(const D
       tnxt = tile_of(i + W);
       rnxt = row_lane(i + W, cnxt);
 #define OGS_LOAD_NXT(D) warp_load_state<MODE, D>(m.b[D], nxt, m.wemask, tnxt, use_mask, pat, rnxt, snxt)
-      OGS_DEGREE_SWITCH(nxt.bucket, OGS_LOAD_NXT)
+      if (LONE && nxt.bucket == kLoneBucket) lone_rows(m, nxt, lane, snxt);
+      else OGS_DEGREE_SWITCH(nxt.bucket, OGS_LOAD_NXT)
 #undef OGS_LOAD_NXT
       if (i + 2 * W < nitems) nn = m.wtiles[tile_of(i + 2 * W)];
     }
 #define OGS_FOLD(D) warp_fold_store<T, OP, MODE, D>(scur, dst, gv, stride, K, k0, gmask, smode, gslib, rcur, V)
-    OGS_DEGREE_SWITCH(cur.bucket, OGS_FOLD)
+    if (LONE && cur.bucket == kLoneBucket) lone_gather<T, OP>(scur, gv, V);
+    else OGS_DEGREE_SWITCH(cur.bucket, OGS_FOLD)
 #undef OGS_FOLD
     if (!more) break;
     i += W;
@@ -246,14 +288,14 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_warp_kernel(const D
 
 
 // CTAs of the warp kernel resident per SM, once per instantiation and device.
-template <typename T, int OP, int MODE, int KL, bool PLAIN>
+template <typename T, int OP, int MODE, int KL, bool PLAIN, bool LONE = false>
 inline int warp_grid(int64_t nitems) {
   static DeviceCache cache;
   int dev = 0;
   cudaGetDevice(&dev);
   const int cached = cache.get(dev, [dev] {
     int bps = 0, sms = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, ogs_warp_kernel<T, OP, MODE, KL, PLAIN>, kBlock, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, ogs_warp_kernel<T, OP, MODE, KL, PLAIN, LONE>, kBlock, 0);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     return (bps > 0 ? bps : 1) * (sms > 0 ? sms : 1);
   });
@@ -261,15 +303,23 @@ inline int warp_grid(int64_t nitems) {
   return static_cast<int>(need < cached ? need : cached);
 }
 
-template <typename T, int OP, int MODE, int KL, bool PLAIN>
+template <typename T, int OP, int MODE, int KL, bool PLAIN, bool LONE = false>
 inline void launch_warp_kl(const DevMaps& m, const FieldArgs& f, Pattern pat, cudaStream_t s) {
   const int64_t nitems = static_cast<int64_t>(m.nwtiles) * (KL == kK1 ? 1 : f.K);
-  const int grid = warp_grid<T, OP, MODE, KL, PLAIN>(nitems);
-  launch_overlapped(ogs_warp_kernel<T, OP, MODE, KL, PLAIN>, grid, kBlock, 0, s, f.overlap, m, f, pat);
+  const int grid = warp_grid<T, OP, MODE, KL, PLAIN, LONE>(nitems);
+  launch_overlapped(ogs_warp_kernel<T, OP, MODE, KL, PLAIN, LONE>, grid, kBlock, 0, s, f.overlap, m, f, pat);
 }
 
 template <typename T, int OP, int MODE, bool PLAIN>
 inline void launch_warp_plain(const DevMaps& m, const FieldArgs& f, Pattern pat, cudaStream_t s) {
+  if constexpr (MODE == kModeGather && PLAIN) {
+    if (f.K == 1 && m.nltiles > 0 && m.nodes.nwords > 0) {
+      DevMaps l = m;
+      l.wtiles = m.ltiles;
+      l.nwtiles = m.nltiles;
+      return launch_warp_kl<T, OP, MODE, kK1, PLAIN, true>(l, f, pat, s);
+    }
+  }
   if (f.is_many) launch_warp_kl<T, OP, MODE, kKMany, PLAIN>(m, f, pat, s);
   else if (f.K == 1) launch_warp_kl<T, OP, MODE, kK1, PLAIN>(m, f, pat, s);
   else launch_warp_kl<T, OP, MODE, kKInterleaved, PLAIN>(m, f, pat, s);

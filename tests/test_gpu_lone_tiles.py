@@ -64,6 +64,29 @@ def test_lone(cuda, oracle_mod, n, dtype):
                 assert same_bits(d.cpu().numpy(), ref.gather_scatter(x.copy(), 1, op, "sym")), (kind, op)
 
 
+@pytest.mark.parametrize("dtype", list(SPECIAL))
+@pytest.mark.parametrize("n", [2, 255, 256, 257, 515, 4100, 70003])
+def test_lone_gathered(cuda, oracle_mod, n, dtype):
+    """Gather on Signed unique handles: a lone node's row follows from its word's first members."""
+    base = mostly_lone(n, seed=n + 1)
+    if not base.any():
+        base[0] = 1
+    ref = oracle_mod.OracleOgs(base.copy(), "signed", unique=True)
+    for maps in ("host", "device"):
+        g = ogs.ogs_t().Setup(n, base.copy(), None, ogs.Signed, ogs.Auto, True, maps=maps)
+        for op in ("add", "mul", "max", "min"):
+            for tname, trans in (("trans", ogs.Trans), ("notrans", ogs.NoTrans)):
+                v = field(n, dtype, op, seed=n)
+                want = np.zeros(ref.Ngather, dtype)
+                with np.errstate(all="ignore"):
+                    ref.gather(want, v, 1, op, tname)
+                gv = torch.zeros(want.size, dtype=torch.from_numpy(v).dtype, device="cuda")
+                g.Gather(gv, torch.from_numpy(v.copy()).cuda(), 1, ogs.Op[op.capitalize()], trans)
+                got = gv.cpu().numpy()
+                ok = ~(np.isnan(got) & np.isnan(want)) if got.dtype.kind == "f" else np.ones(want.size, bool)
+                assert same_bits(got[ok], want[ok]), (maps, op, tname, first_diff(got, want))
+
+
 def test_signed_patterns_and_host_buffers(cuda, oracle_mod):
     """Handles with lone tiles keep the other tiles for masked patterns and host buffers."""
     ids = signed_ids(mostly_lone(70003, seed=1), seed=4)
