@@ -206,46 +206,64 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_warp_kernel(const D
   const int lane = static_cast<int>(threadIdx.x) & 31;
   const int64_t W = static_cast<int64_t>(gridDim.x) * (kBlock / 32);
   const int K = KL == kK1 ? 1 : f.K;
-  const int64_t nw = m.nwtiles;
-  const int64_t nitems = nw * K;
-  int64_t i = static_cast<int64_t>(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5);
+  const int nw = m.nwtiles;
+  const int64_t i0 = static_cast<int64_t>(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5);
+  const bool idle = i0 >= static_cast<int64_t>(nw) * K;
   grid_release();
   constexpr bool kLate = PLAIN && KL == kK1;
-  if (!kLate || i >= nitems) grid_wait();
-  if (i >= nitems) return;
+  if (!kLate || idle) grid_wait();
+  if (idle) return;
   const bool use_mask = !PLAIN && (pat.gather_n || pat.scatter_n) && m.signed_maps;
   const bool gmask = !PLAIN && pat.gather_n != 0;
   const int smode = PLAIN ? 0 : pat.scatter_n;
   const bool gslib = !PLAIN && pat.gslib != 0;
   const ByteStride stride{(KL == kKInterleaved ? static_cast<uint32_t>(K) : 1u) * static_cast<uint32_t>(sizeof(T))};
-  auto tile_of = [&](int64_t item) {
-    return static_cast<int>(KL == kKMany ? item % nw : (KL == kKInterleaved ? item / K : item));
+  // Items as (tile, part) or, for separate arrays, (tile, array) pairs, advanced
+  // by W without division (as in ogs_async.cuh).
+  struct Pos {
+    int t, c;
   };
+  const int M = KL == kKMany ? nw : (KL == kKInterleaved ? K : 1);
+  const int Wi = static_cast<int>(W), Wq = KL == kK1 ? Wi : Wi / M, Wr = KL == kK1 ? 0 : Wi % M;
+  auto after = [&](Pos p) {
+    if (KL == kK1) return Pos{p.t + Wi, 0};
+    if (KL == kKInterleaved) return p.c + Wr >= M ? Pos{p.t + Wq + 1, p.c + Wr - M} : Pos{p.t + Wq, p.c + Wr};
+    return p.t + Wr >= M ? Pos{p.t + Wr - M, p.c + Wq + 1} : Pos{p.t + Wr, p.c + Wq};
+  };
+  auto valid = [&](Pos p) { return KL == kKMany ? p.c < K : p.t < nw; };
   // k > 1 interleaved: item (tile, part j); thread t works row lane
   // (32j + t) / k, component (32j + t) % k, as in the cp.async pipeline
   const uint32_t kmagic = KL == kKInterleaved && K > 1 ? 0xFFFFFFFFu / static_cast<uint32_t>(K) + 1u : 0u;
-  auto row_lane = [&](int64_t item, int& comp) {
+  auto row_lane = [&](Pos p, int& comp) {
     if (KL != kKInterleaved) {
-      comp = KL == kKMany ? static_cast<int>(item / nw) : 0;
+      comp = p.c;
       return lane;
     }
-    const uint32_t u = static_cast<uint32_t>(item % K) * 32u + static_cast<uint32_t>(lane);
+    const uint32_t u = static_cast<uint32_t>(p.c) * 32u + static_cast<uint32_t>(lane);
     const int rl = static_cast<int>(K < 11585 ? __umulhi(u, kmagic) : u / static_cast<uint32_t>(K));
     comp = static_cast<int>(u) - rl * K;
     return rl;
   };
 
-  int tcur = tile_of(i);
-  Tile cur = m.wtiles[tcur];
+  const int outer = KL == kK1 ? static_cast<int>(i0) : static_cast<int>(i0 / M);
+  const int inner = KL == kK1 ? 0 : static_cast<int>(i0 - static_cast<int64_t>(outer) * M);
+  Pos pcur = KL == kKMany ? Pos{inner, outer} : Pos{outer, inner};
+  Tile cur = m.wtiles[pcur.t];
   WarpState scur;
   int ccur;
-  int rcur = row_lane(i, ccur);
-#define OGS_LOAD_CUR(D) warp_load_state<MODE, D>(m.b[D], cur, m.wemask, tcur, use_mask, pat, rcur, scur)
+  int rcur = row_lane(pcur, ccur);
+#define OGS_LOAD_CUR(D) warp_load_state<MODE, D>(m.b[D], cur, m.wemask, pcur.t, use_mask, pat, rcur, scur)
   if (LONE && cur.bucket == kLoneBucket) lone_rows(m, cur, lane, scur);
   else OGS_DEGREE_SWITCH(cur.bucket, OGS_LOAD_CUR)
 #undef OGS_LOAD_CUR
   Tile nxt{};
-  if (i + W < nitems) nxt = m.wtiles[tile_of(i + W)];
+  // (k = 1 counts items: carrying the next positions there made a Gather 24^3
+  // p=15 fp64 166 us instead of 162)
+  const int64_t nitems = static_cast<int64_t>(nw) * K;
+  int64_t i = i0;
+  Pos pnxt = after(pcur);
+  bool ahead = KL != kK1 && valid(pnxt);
+  if (KL == kK1 ? i + W < nitems : ahead) nxt = m.wtiles[pnxt.t];
 
   T* gv = static_cast<T*>(f.gv);
   if (kLate) grid_wait();  // (as in ogs_async.cuh)
@@ -258,18 +276,24 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_warp_kernel(const D
     if (LONE && cur.bucket == kLoneBucket) lone_load_vals(scur, src, lane, V);
     else OGS_DEGREE_SWITCH(cur.bucket, OGS_VALS)
 #undef OGS_VALS
-    const bool more = i + W < nitems;
+    const bool more = KL == kK1 ? i + W < nitems : ahead;
     WarpState snxt;
     Tile nn{};
-    int tnxt = 0, cnxt = 0, rnxt = lane;
+    Pos pnn{};
+    int cnxt = 0, rnxt = lane;
     if (more) {
-      tnxt = tile_of(i + W);
-      rnxt = row_lane(i + W, cnxt);
-#define OGS_LOAD_NXT(D) warp_load_state<MODE, D>(m.b[D], nxt, m.wemask, tnxt, use_mask, pat, rnxt, snxt)
+      rnxt = row_lane(pnxt, cnxt);
+#define OGS_LOAD_NXT(D) warp_load_state<MODE, D>(m.b[D], nxt, m.wemask, pnxt.t, use_mask, pat, rnxt, snxt)
       if (LONE && nxt.bucket == kLoneBucket) lone_rows(m, nxt, lane, snxt);
       else OGS_DEGREE_SWITCH(nxt.bucket, OGS_LOAD_NXT)
 #undef OGS_LOAD_NXT
-      if (i + 2 * W < nitems) nn = m.wtiles[tile_of(i + 2 * W)];
+      if (KL == kK1) {
+        if (i + 2 * W < nitems) nn = m.wtiles[i + 2 * W];
+      } else {
+        pnn = after(pnxt);
+        ahead = valid(pnn);
+        if (ahead) nn = m.wtiles[pnn.t];
+      }
     }
 #define OGS_FOLD(D) warp_fold_store<T, OP, MODE, D>(scur, dst, gv, stride, K, k0, gmask, smode, gslib, rcur, V)
     if (LONE && cur.bucket == kLoneBucket) lone_gather<T, OP>(scur, gv, V);
@@ -280,7 +304,7 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_warp_kernel(const D
     cur = nxt;
     scur = snxt;
     nxt = nn;
-    tcur = tnxt;
+    pnxt = KL == kK1 ? Pos{static_cast<int>(i + W), 0} : pnn;
     ccur = cnxt;
     rcur = rnxt;
   }

@@ -70,6 +70,27 @@ def test_chains(cuda, sizes, k):
         assert torch.equal(q, want) and torch.equal(gv, wgv)
 
 
+@pytest.mark.parametrize("n,k", [(2000, 1), (60000, 1), (60000, 3), (900000, 1)])
+def test_chains_with_general_rows(cuda, n, k):
+    """Two launches a call: about half the nodes in rows of degree 20."""
+    ids = mesh.uniform_values(n, np.int64, 1, 1 + n // 40, 6)
+    few = mesh.uniform_values(n, np.int64, 0, 2, 7) == 0
+    ids[few] = n + mesh.uniform_values(int(few.sum()), np.int64, 1, 1 + n // 4, 8)
+    g = ogs.ogs_t().Setup(ids.size, ids.copy(), None, ogs.Signed, ogs.Auto, True)
+    assert g.max_degree > 8
+    ref = Rows(ids, k)
+    v = torch.from_numpy(mesh.uniform_values(k * n, np.int64, -1000, 1000, 9)).cuda()
+    want, wgv = v.clone(), torch.zeros(k * g.Ngather, dtype=torch.int64, device="cuda")
+    chain(g, ref, want, wgv, k, 12)
+    for stream in (torch.cuda.current_stream(), torch.cuda.Stream()):
+        torch.cuda.synchronize()
+        with torch.cuda.stream(stream):
+            q, gv = v.clone(), torch.zeros_like(wgv)
+            chain(g, None, q, gv, k, 12)
+        torch.cuda.synchronize()
+        assert torch.equal(q, want) and torch.equal(gv, wgv)
+
+
 def test_two_streams(cuda):
     """A field handed back and forth between two streams by events, each with work of its own queued."""
     ids, g = handle((12, 11, 10, 4))
