@@ -25,7 +25,7 @@
 // ogs_get_maps.  Both paths give identical handles.
 //
 // Every buffer here is scratch of the setup call and is freed before it
-// returns.  Device memory needed: about 70 bytes per local node.
+// returns.  Device memory needed: 78 bytes per local node (91 Signed).
 #include <algorithm>
 #include <cstdint>
 #include <limits>
@@ -428,21 +428,45 @@ __global__ void k_node_others(const int32_t* __restrict__ code, const int32_t* _
   if ((other >> lane) & 1u) orow[o + __popc(other & ((1u << lane) - 1u))] = ~code[n];
 }
 
-// Device scratch of one setup call, freed on every exit path.
+// Device scratch of one setup call, freed on every exit path: pieces of one
+// block (an allocation or a free of its own costs each piece 40 us of host time,
+// the block 85 and 265), and allocations of their own beyond it.  The pieces
+// from a mark on can be given up for others once the work that uses them is
+// queued: all of it runs on one stream.
 struct Scratch {
   std::vector<void*> bufs;
+  char* block = nullptr;
+  size_t size = 0, used = 0;
   ~Scratch() {
     for (void* p : bufs) dev_free(p);
   }
+  static size_t padded(size_t bytes) { return (std::max<size_t>(bytes, 1) + 255) / 256 * 256; }
+  cudaError_t reserve(size_t bytes) {
+    const cudaError_t e = dev_malloc(&block, bytes);
+    if (e != cudaSuccess) {
+      block = nullptr;
+      return e;
+    }
+    bufs.push_back(block);
+    size = bytes;
+    return e;
+  }
   template <typename T>
   cudaError_t get(T** p, int64_t count) {
+    const size_t bytes = padded(static_cast<size_t>(count > 0 ? count : 1) * sizeof(T));
+    if (used + bytes <= size) {
+      *p = reinterpret_cast<T*>(block + used);
+      used += bytes;
+      return cudaSuccess;
+    }
     void* q = nullptr;
-    const size_t bytes = static_cast<size_t>(count > 0 ? count : 1) * sizeof(T);
     const cudaError_t e = dev_malloc(&q, bytes);
     if (e == cudaSuccess) bufs.push_back(q);
     *p = static_cast<T*>(q);
     return e;
   }
+  size_t mark() const { return used; }
+  void rewind(size_t m) { used = m; }
 };
 
 template <typename T>
@@ -467,8 +491,15 @@ cudaError_t inclusive_sum(Scratch& sc, const T* in, T* out, int64_t n, cudaStrea
 
 }  // namespace
 
+namespace {
+
+// The maps' layout from the device CSR maps: the arena, DevMaps and the
+// host-side tile lists and phases.  code: per node its row (a first member),
+// ~row (another member) or INT32_MIN; nmem: per node whether it is an N member
+// (both only read when the handle gets node words).
 ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_t* ciT, const int32_t* rsN,
-                               const int32_t* ciN, const int32_t* code, const uint8_t* nmem, void* stream) {
+                               const int32_t* ciN, const int32_t* code, const uint8_t* nmem, Scratch& sc,
+                               void* stream) {
   TraceRange trace("ogs_setup: layout on the GPU");
   const cudaStream_t st = static_cast<cudaStream_t>(stream);
   HostLayout& L = h->lay;
@@ -479,7 +510,6 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
     rsN = rsT;
     ciN = ciT;
   }
-  Scratch sc;
   auto fail = [&](cudaError_t e, const char* what) {
     cudaGetLastError();
     return set_error(e == cudaErrorMemoryAllocation ? OGS_ENOMEM : OGS_EDEVICE,
@@ -794,6 +824,8 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
   return OGS_OK;
 }
 
+}  // namespace
+
 ogs_status build_device_maps(ogs_handle_s* h, int64_t N, int64_t* ids, int kind, int unique, bool layout) {
   TraceRange trace("ogs_setup: maps on the GPU");
   if (kind == OGS_HALO)
@@ -832,28 +864,38 @@ ogs_status build_device_maps(ogs_handle_s* h, int64_t N, int64_t* ids, int kind,
   };
 
   // 1. keys and a stable sort by |id|
+  // The block: ids, maps and node codes first, which live to the end, then what
+  // the maps are made from, and the sorts' own scratch (about 2 bytes a node).
   int64_t* d_ids = nullptr;
   uint64_t *key = nullptr, *key2 = nullptr;
   int32_t *val = nullptr, *val2 = nullptr;
   Counters* d_c = nullptr;
-  cudaError_t e = sc.get(&d_ids, N);
-  if (!e) e = sc.get(&key, N);
-  if (!e) e = sc.get(&key2, N);
-  if (!e) e = sc.get(&val, N);
-  if (!e) e = sc.get(&val2, N);
+  const size_t n1 = static_cast<size_t>(N) + 1;
+  const size_t live = Scratch::padded(n1 * 8) + 3 * Scratch::padded(n1 * 4) +
+                      (sgn ? 2 * Scratch::padded(n1 * 4) + Scratch::padded(n1) : 0);
+  const size_t made = 3 * Scratch::padded(n1 * 8) + 8 * Scratch::padded(n1 * 4);
+  cudaError_t e = sc.reserve(live + made + n1 * 2 + (8 << 20));
+  if (!e) e = sc.get(&d_ids, N);
+  int32_t *rsT = nullptr, *rsN = nullptr, *ciT = nullptr, *ciN = nullptr;
+  if (!e) e = sc.get(&rsT, N + 1);
+  if (!e) e = sc.get(&rsN, N + 1);
+  if (!e) e = sc.get(&ciT, N);
+  if (!e && sgn) e = sc.get(&ciN, N);
+  // whether the handle gets node words is not known yet: Signed ones may
+  int32_t* code = nullptr;
+  uint8_t* nmem = nullptr;
+  if (!e && sgn && layout) e = sc.get(&code, N);
+  if (!e && sgn && layout) e = sc.get(&nmem, N);
   if (!e) e = sc.get(&d_c, 1);
+  const size_t kept = sc.mark();
+  if (!e) e = sc.get(&key, N + 1);
+  if (!e) e = sc.get(&key2, N + 1);
+  if (!e) e = sc.get(&val, N + 1);
+  if (!e) e = sc.get(&val2, N + 1);
   if (e) return fail(e, "allocation");
   e = cudaMemcpyAsync(d_ids, ids, static_cast<size_t>(N) * sizeof(int64_t), cudaMemcpyHostToDevice, st);
   if (!e) e = cudaMemsetAsync(d_c, 0, sizeof(Counters), st);
   if (e) return fail(e, "copy in");
-  // whether the handle gets node words is not known yet: Signed ones may
-  int32_t* code = nullptr;
-  uint8_t* nmem = nullptr;
-  if (sgn && layout) {
-    e = sc.get(&code, N);
-    if (!e) e = sc.get(&nmem, N);
-    if (e) return fail(e, "allocation");
-  }
   k_keys<<<rblocks(N), kT, 0, st>>>(d_ids, N, key, val, code, d_c);
   Counters c{};
   e = cudaMemcpyAsync(&c, d_c, sizeof(Counters), cudaMemcpyDeviceToHost, st);
@@ -866,23 +908,26 @@ ogs_status build_device_maps(ogs_handle_s* h, int64_t N, int64_t* ids, int kind,
   if (nnz == 0) return empty_maps();
   int end_bit = 1;
   while (end_bit < 64 && (c.maxkey >> end_bit) != 0) end_bit++;
+  cub::DoubleBuffer<uint64_t> keys(key, key2);
+  cub::DoubleBuffer<int32_t> vals(val, val2);
   {
     size_t bytes = 0;
-    e = cub::DeviceRadixSort::SortPairs(nullptr, bytes, key, key2, val, val2, N, 0, end_bit, st);
+    e = cub::DeviceRadixSort::SortPairs(nullptr, bytes, keys, vals, N, 0, end_bit, st);
     char* tmp = nullptr;
     if (!e) e = sc.get(&tmp, static_cast<int64_t>(bytes));
-    if (!e) e = cub::DeviceRadixSort::SortPairs(tmp, bytes, key, key2, val, val2, N, 0, end_bit, st);
+    if (!e) e = cub::DeviceRadixSort::SortPairs(tmp, bytes, keys, vals, N, 0, end_bit, st);
     if (e) return fail(e, "sort");
   }
-  const uint64_t* skey = key2 + zeros;  // zero ids sort first
-  const int32_t* sval = val2 + zeros;
+  const uint64_t* skey = keys.Current() + zeros;  // zero ids sort first
+  const int32_t* sval = vals.Current() + zeros;
 
-  // 2. heads, group numbers, positive members before each member
-  int32_t *head = nullptr, *gincl = nullptr, *pos = nullptr, *pos_ex = nullptr;
-  e = sc.get(&head, nnz);
-  if (!e) e = sc.get(&gincl, nnz);
-  if (!e) e = sc.get(&pos, nnz + 1);
-  if (!e) e = sc.get(&pos_ex, nnz + 1);
+  // 2. heads, group numbers, positive members before each member, in the other
+  // buffers of the sort
+  int32_t* const head = reinterpret_cast<int32_t*>(keys.Alternate());
+  int32_t* const gincl = head + N;
+  int32_t* const pos = vals.Alternate();
+  int32_t* pos_ex = nullptr;
+  e = sc.get(&pos_ex, nnz + 1);
   if (e) return fail(e, "allocation");
   e = cudaMemsetAsync(pos + nnz, 0, sizeof(int32_t), st);
   if (e) return fail(e, "memset");
@@ -897,14 +942,14 @@ ogs_status build_device_maps(ogs_handle_s* h, int64_t N, int64_t* ids, int kind,
 
   // 3. per-group figures and first-appearance ranks
   int32_t *gstart = nullptr, *gfirst = nullptr, *gsize = nullptr, *gpos = nullptr, *grow = nullptr;
-  uint64_t *mark = nullptr, *rank = nullptr;
+  uint64_t* mark = nullptr;
+  uint64_t* const rank = keys.Current();  // the sorted keys have given their heads
   e = sc.get(&gstart, ngroups + 1);
   if (!e) e = sc.get(&gfirst, ngroups);
   if (!e) e = sc.get(&gsize, ngroups);
   if (!e) e = sc.get(&gpos, ngroups);
   if (!e) e = sc.get(&grow, ngroups);
   if (!e) e = sc.get(&mark, N + 1);
-  if (!e) e = sc.get(&rank, N + 1);
   if (e) return fail(e, "allocation");
   const int32_t nnz32 = static_cast<int32_t>(nnz);
   e = cudaMemcpyAsync(gstart + ngroups, &nnz32, sizeof(int32_t), cudaMemcpyHostToDevice, st);
@@ -921,14 +966,8 @@ ogs_status build_device_maps(ogs_handle_s* h, int64_t N, int64_t* ids, int kind,
   const int64_t nlocalP = static_cast<int64_t>(total & 0xffffffffu);
 
   // 4. rows, row starts, members into place
-  int32_t *degT = nullptr, *degN = nullptr, *rsT = nullptr, *rsN = nullptr, *ciT = nullptr, *ciN = nullptr;
-  e = sc.get(&degT, ngroups + 1);
-  if (!e) e = sc.get(&degN, ngroups + 1);
-  if (!e) e = sc.get(&rsT, ngroups + 1);
-  if (!e) e = sc.get(&rsN, ngroups + 1);
-  if (!e) e = sc.get(&ciT, nnz);
-  if (!e && sgn) e = sc.get(&ciN, nnz);
-  if (e) return fail(e, "allocation");
+  int32_t* const degT = reinterpret_cast<int32_t*>(mark);  // ranked
+  int32_t* const degN = degT + (ngroups + 1);
   e = cudaMemsetAsync(degT + ngroups, 0, sizeof(int32_t), st);
   if (!e) e = cudaMemsetAsync(degN + ngroups, 0, sizeof(int32_t), st);
   if (e) return fail(e, "memset");
@@ -949,7 +988,8 @@ ogs_status build_device_maps(ogs_handle_s* h, int64_t N, int64_t* ids, int kind,
   h->nnzT = nnz;
   // the kernels' layout, built from the maps while they are on the device
   if (layout) {
-    ogs_status ls = build_device_layout(h, rsT, ciT, sgn ? rsN : nullptr, sgn ? ciN : nullptr, code, nmem, st);
+    sc.rewind(kept);
+    ogs_status ls = build_device_layout(h, rsT, ciT, sgn ? rsN : nullptr, sgn ? ciN : nullptr, code, nmem, sc, st);
     if (ls != OGS_OK) return ls;
   }
   // maps back to the host

@@ -339,13 +339,6 @@ void build_layout(ogs_handle_s* h);
 ogs_status upload_layout(ogs_handle_s* h);
 void release_device(ogs_handle_s* h);
 void build_phases(ogs_handle_s* h, int max_phases);  // needs the tiles and their lo/hi
-// The maps' layout built on the current device from device CSR maps
-// (ogs_dsetup.cu): the arena, DevMaps and the host-side tile lists and phases.
-// d_code: per node its row (a first member), ~row (another member) or
-// INT32_MIN; d_nmem: per node whether it is an N member (both only read when
-// the handle gets node words).
-ogs_status build_device_layout(ogs_handle_s* h, const int32_t* d_rsT, const int32_t* d_ciT, const int32_t* d_rsN,
-                               const int32_t* d_ciN, const int32_t* d_code, const uint8_t* d_nmem, void* stream);
 // Whether a handle gets node words: Scatter is defined and every row has a
 // positive member, so that rows are numbered by first member.
 inline bool wants_node_words(const ogs_handle_s* h) {
