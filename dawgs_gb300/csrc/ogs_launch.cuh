@@ -3,8 +3,8 @@
 // Scatter runs in node order where the handle's rows are numbered by first
 // member (ogs_scatter.cuh).  Otherwise exact-degree rows of GatherScatter run
 // on the warp pipeline with cp.async-staged gathers (ogs_async.cuh), those of
-// Gather and Scatter on the register pipeline of ogs_warp.cuh
-// (-DOGS_GATHER_REGISTERS=0: everything on the cp.async one; -DOGS_ASYNC=0:
+// Gather, and of Scatter over rows in another order, on the register pipeline
+// of ogs_warp.cuh (-DOGS_GATHER_REGISTERS=0: everything on the cp.async one; -DOGS_ASYNC=0:
 // everything on the register one).  Rows above degree 8 run as wide tiles
 // (ogs_wide.cuh), or on the direct CTA kernel (ogs_kernels.cuh).  Building
 // with -DOGS_KERNEL=2 runs the direct CTA kernel for every row instead (for
@@ -13,8 +13,8 @@
 // Why the split: a GatherScatter row is read and written in place, and two
 // tiles' gathers in flight through the shared-memory ring beat one in
 // registers (24^3 p=7 fp64: 28.3 vs 31.6 us; 32x32x16 p=5 permuted k=3: 41.1
-// vs 42.4 us); a Gather writes one value per row and a Scatter reads one per
-// row, and there the ring's shared-memory fills cost more than they hide
+// vs 42.4 us); a Gather writes one value per row and a Scatter in row order
+// reads one per row, and there the ring's shared-memory fills cost more than they hide
 // (24^3 p=7: Gather Trans 25.2 vs 26.6 us, Scatter NoTrans 29.9 vs 30.6 us;
 // k=3: Gather 32.9 vs 52.0 us, Scatter 47.3 vs 50.9 us).
 #pragma once
