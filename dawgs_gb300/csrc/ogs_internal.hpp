@@ -250,6 +250,21 @@ struct FieldArgs {
   int32_t overlap = 0;      // host: launch with programmatic stream serialization
 };
 
+// Whether a Scatter runs in node order (ogs_scatter.cuh): where the handle has
+// node words (rows numbered by first member), for up to kScatterMaxK components.
+// A warp takes every component of a word, so more of them leave a small mesh
+// with few warps that each go through many rounds (eight runs a round: 1,000
+// nodes k=1000 117 us against 3.9 through the column lists, 64 nodes k=20000
+// 2,459 against 7.9, 20^3 p=7 k=64 fp64 93 against 78, k=16 27.6 against 23.0).
+// Up to eight it is the faster one on boxes from 6^3 p=3 to 24^3 p=7, permuted
+// or not, fp32 and fp64 (0.55 to 1.0 of the time) but for fp64 k=4 and fp32 k=5
+// at 24^3 p=7 (74.1 and 61.2 us against 70.5 and 58.2).  Operators over caller
+// maps and the slices of host-buffer calls keep the tile kernels.
+constexpr int kScatterMaxK = 8;
+inline bool scatter_applies(const DevMaps& m, const FieldArgs& f, const Pattern& pat) {
+  return m.nodes.nwords > 0 && f.K <= kScatterMaxK && !f.is_many && !pat.gslib && pat.scatter_n <= 1;
+}
+
 // A slice of the warp and general tiles for the host-buffer pipeline: its
 // kernels read and write local nodes in [lo, hi]; its host->device chunk is
 // [h0, h1) and once it has run, local nodes [d0, d1) are final and go back.

@@ -1,0 +1,35 @@
+"""The rules that choose a call's kernel, compiled for the host: what they accept
+stays within what the chosen kernel's index arithmetic holds."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from dawgs_gb300 import build
+
+pytestmark = pytest.mark.skipif(shutil.which("g++") is None, reason="needs g++")
+
+
+def run(tmp_path, body):
+    """The words that a program printing `body`'s results writes."""
+    src, exe = tmp_path / "rules.cpp", tmp_path / "rules"
+    src.write_text('#include <cstdio>\n#include "ogs_internal.hpp"\nusing namespace ogsgb;\n'
+                   "void out(long long x) { std::printf(\"%lld \", x); }\nint main() {\n" + body + "\n}\n")
+    cuda = os.path.dirname(os.path.dirname(build.nvcc()))
+    r = subprocess.run(["g++", "-std=c++17", "-I", build.INCLUDE, "-I", build.CSRC, "-I",
+                        os.path.join(cuda, "include"), str(src), "-o", str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    return [int(x) for x in subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout.split()]
+
+
+KS = [1, 2, 8, 9, 64, 1000, 2**26, 2**26 + 1, 2**27, 2**27 + 1, 2**31 - 1]
+
+
+def test_scatter_in_node_order_takes_few_components(tmp_path):
+    """A warp walks every component of its nodes, so large k goes to the tiles;
+    no accepted k brings a component's place in a word near 32 bits."""
+    body = "DevMaps m{}; m.nodes.nwords = 40; FieldArgs f{}; Pattern p{0, 0, 0};\n"
+    body += "".join(f"f.K = {k}; out(scatter_applies(m, f, p));\n" for k in KS)
+    got = run(tmp_path, body)
+    assert got == [1, 1, 1] + [0] * 8
