@@ -23,7 +23,15 @@
 
 namespace ogsgb {
 
-constexpr int kScatterBlock = 256;
+// Threads of a CTA: 256, or 64 where that makes fewer than kScatterCtas CTAs
+// (3.4 an SM), since a small mesh leaves SMs idle and CTAs of 64 for 7 M nodes
+// take as long as 55 k CTAs need to start.  CTAs of 256 / of 64 / through the
+// column lists, us: fp64 k=2 10^3 p=3 (64 k nodes) 3.00 / 2.85 / 2.87, k=4 2.96 /
+// 2.75 / 2.69, k=1 2.97 / 2.90 / 2.87, 24^3 p=3 4.23 / 4.16 / 4.64; the other
+// way fp32 k=1 24^3 p=7 10.8 / 14.7, k=3 16^3 p=3 (512 CTAs) 2.75 / 2.87, 24^3
+// p=7 34.9 / 56.5.
+constexpr int kScatterBlock = 256, kScatterSmallBlock = 64;
+constexpr int64_t kScatterCtas = 512;
 
 // Words of 32 nodes a warp takes for K components, all their loads in flight at
 // once: about eight runs of 32 values.
@@ -37,7 +45,7 @@ __global__ void __launch_bounds__(kScatterBlock) ogs_scatter_kernel(const DevNod
                                                                     const int32_t nrows, unsigned int* err) {
   constexpr int W = scatter_words(K);
   const int lane = static_cast<int>(threadIdx.x) & 31;
-  const int64_t w0 = (static_cast<int64_t>(blockIdx.x) * (kScatterBlock / 32) + (threadIdx.x >> 5)) * W;
+  const int64_t w0 = (static_cast<int64_t>(blockIdx.x) * (blockDim.x / 32) + (threadIdx.x >> 5)) * W;
   grid_release();
   if (w0 >= m.nwords) {
     grid_wait();
@@ -76,9 +84,13 @@ __global__ void __launch_bounds__(kScatterBlock) ogs_scatter_kernel(const DevNod
 
 template <typename T, int K, bool NONLY>
 inline cudaError_t launch_scatter_as(const DevMaps& m, const FieldArgs& f, cudaStream_t s) {
-  constexpr int64_t per_block = scatter_words(K) * (kScatterBlock / 32);
-  const unsigned grid = static_cast<unsigned>((m.nodes.nwords + per_block - 1) / per_block);
-  return launch_overlapped(ogs_scatter_kernel<T, K, NONLY>, dim3(grid), kScatterBlock, 0, s, f.overlap, m.nodes,
+  auto ctas = [&](int block) {
+    const int64_t per_block = scatter_words(K) * (block / 32);
+    return (m.nodes.nwords + per_block - 1) / per_block;
+  };
+  const int block = ctas(kScatterBlock) < kScatterCtas ? kScatterSmallBlock : kScatterBlock;
+  const dim3 grid(static_cast<unsigned>(ctas(block)));
+  return launch_overlapped(ogs_scatter_kernel<T, K, NONLY>, grid, block, 0, s, f.overlap, m.nodes,
                            static_cast<T*>(f.v), static_cast<const T*>(f.gv), m.b[1].nrows, m.b[1].err);
 }
 
