@@ -864,6 +864,7 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
   m.nodes.nmem = reinterpret_cast<const uint32_t*>(base + o_nmem);
   m.nodes.orow = reinterpret_cast<const int32_t*>(base + o_orow);
   m.nodes.nwords = nwords;
+  m.nodes.scatter = nwords > 0 && scatter_share(h);
   m.signed_maps = sgn ? 1 : 0;
   set_id_bounds(h, m, reinterpret_cast<unsigned int*>(base + o_err));
   return OGS_OK;

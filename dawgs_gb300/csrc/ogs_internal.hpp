@@ -181,6 +181,7 @@ struct DevNodes {
   const uint32_t* nmem;   // bit per node: in the N map (padded alike)
   const int32_t* orow;
   int64_t nwords;         // 0: the handle has none
+  int32_t scatter;        // whether a Scatter runs over them (scatter_share)
 };
 constexpr int kNodeWordPad = 16;
 inline int64_t node_words(int64_t N) { return (N + 31) / 32; }
@@ -251,7 +252,8 @@ struct FieldArgs {
 };
 
 // Whether a Scatter runs in node order (ogs_scatter.cuh): where the handle has
-// node words (rows numbered by first member), for up to kScatterMaxK components.
+// node words (rows numbered by first member) and most of its nodes take part
+// (scatter_share), for up to kScatterMaxK components.
 // A warp takes every component of a word, so more of them leave a small mesh
 // with few warps that each go through many rounds (eight runs a round: 1,000
 // nodes k=1000 117 us against 3.9 through the column lists, 64 nodes k=20000
@@ -262,7 +264,7 @@ struct FieldArgs {
 // maps and the slices of host-buffer calls keep the tile kernels.
 constexpr int kScatterMaxK = 8;
 inline bool scatter_applies(const DevMaps& m, const FieldArgs& f, const Pattern& pat) {
-  return m.nodes.nwords > 0 && f.K <= kScatterMaxK && !f.is_many && !pat.gslib && pat.scatter_n <= 1;
+  return m.nodes.scatter && f.K <= kScatterMaxK && !f.is_many && !pat.gslib && pat.scatter_n <= 1;
 }
 
 // A slice of the warp and general tiles for the host-buffer pipeline: its
@@ -360,6 +362,13 @@ inline bool wants_node_words(const ogs_handle_s* h) {
   return h->kind == OGS_SIGNED && h->gather_defined && !h->from_maps && !h->gslib && h->NlocalT > 0 &&
          h->NlocalP == h->NlocalT;
 }
+// Whether enough nodes take part for a Scatter to go through all of them: three
+// quarters.  In 10 M nodes of which the first part takes part, pairs of
+// neighbours, fp64 k=3, through the column lists / in node order: 1/2 37.0 /
+// 43.8 us, 5/8 45.1 / 49.1, 3/4 53.0 / 54.2, 7/8 60.7 / 59.0; 1/1000 of 7 M
+// nodes 2.5 / 15.4.  (Parts that lie between the others do better: 1/2 89.4 /
+// 81.0.)
+inline bool scatter_share(const ogs_handle_s* h) { return h->nnzT * 4 >= h->N * 3; }
 // Wide tiles of general rows with the given row starts; the units of 32 ids
 // they take.  None where rows of very different degree are neighbours and the
 // padding would outweigh the rows.

@@ -560,6 +560,7 @@ DevMaps general_maps(const DevMaps& m) {
 // copies of a sliced host-buffer call set its time.
 DevMaps phase_maps(const DevMaps& m, const Phase& p) {
   DevMaps r = m;
+  r.nodes.scatter = 0;
   r.nodes.nwords = 0;
   r.nwide = r.nltiles = 0;
   r.wtiles = m.wtiles + p.w0;
@@ -699,6 +700,7 @@ ogs_status upload_layout(ogs_handle_s* h) {
   m.nodes.nmem = reinterpret_cast<const uint32_t*>(base + o_nmem);
   m.nodes.orow = reinterpret_cast<const int32_t*>(base + o_orow);
   m.nodes.nwords = L.nwords.empty() ? 0 : node_words(h->N);
+  m.nodes.scatter = m.nodes.nwords > 0 && scatter_share(h);
   set_id_bounds(h, m, reinterpret_cast<unsigned int*>(base + o_err));
 
   m.signed_maps = sgn ? 1 : 0;

@@ -29,3 +29,12 @@ def test_at_the_larger_ctas(cuda, oracle_mod, k, words, more):
     n = 511 * words * 32 + more
     for dtype in (np.float64, np.float32):
         scattered(oracle_mod, random_ids(n, n // 3, seed=n, zero_frac=0.1), k, dtype)
+
+
+@pytest.mark.parametrize("k", [1, 3, 9])
+@pytest.mark.parametrize("zeros", [0.22, 0.28, 0.99])
+def test_where_few_nodes_take_part(cuda, oracle_mod, zeros, k):
+    """Both sides of the share of nodes from which a Scatter runs in node order."""
+    n = 70001
+    ids = random_ids(n, n // 3, seed=k, zero_frac=zeros)
+    scattered(oracle_mod, ids, k, np.float64)

@@ -29,7 +29,14 @@ KS = [1, 2, 8, 9, 64, 1000, 2**26, 2**26 + 1, 2**27, 2**27 + 1, 2**31 - 1]
 def test_scatter_in_node_order_takes_few_components(tmp_path):
     """A warp walks every component of its nodes, so large k goes to the tiles;
     no accepted k brings a component's place in a word near 32 bits."""
-    body = "DevMaps m{}; m.nodes.nwords = 40; FieldArgs f{}; Pattern p{0, 0, 0};\n"
+    body = "DevMaps m{}; m.nodes.nwords = 40; m.nodes.scatter = 1; FieldArgs f{}; Pattern p{0, 0, 0};\n"
     body += "".join(f"f.K = {k}; out(scatter_applies(m, f, p));\n" for k in KS)
     got = run(tmp_path, body)
     assert got == [1, 1, 1] + [0] * 8
+
+
+def test_scatter_in_node_order_takes_handles_with_most_nodes_in_rows(tmp_path):
+    """Its time goes with all nodes, that of the column lists with those in rows."""
+    body = "ogs_handle_s h; h.N = 1000;\n"
+    body += "".join(f"h.nnzT = {n}; out(scatter_share(&h));\n" for n in (1, 500, 749, 750, 1000))
+    assert run(tmp_path, body) == [0, 0, 0, 1, 1]
