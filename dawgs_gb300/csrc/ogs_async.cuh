@@ -150,13 +150,13 @@ __device__ __forceinline__ void lone_issue(const WarpState& s, const T* src, int
   for (int j = 0; j < 8 / VEC; ++j) {
     const int at = (j * 32 + lane) * VEC;
     if (!((s.emask >> (j * VEC)) & ((1u << VEC) - 1u))) continue;
-    if (s.I[0] + at + VEC <= N) {
+    if (lone_vector_in(s.I[0], at, VEC, N)) {
       const unsigned to = static_cast<unsigned>(__cvta_generic_to_shared(stage + at));
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(to), "l"(src + s.I[0] + at) : "memory");
     } else {  // the field's last vector
 #pragma unroll
       for (int i = 0; i < VEC; ++i)
-        if (s.I[0] + at + i < N) cp_async_elem(stage + at + i, src + s.I[0] + at + i);
+        if (lone_vector_in(s.I[0], at + i, 1, N)) cp_async_elem(stage + at + i, src + s.I[0] + at + i);
     }
   }
 }

@@ -195,6 +195,9 @@ constexpr int kLoneBucket = kDmax + 1;
 // Bit q of lane l's byte stands for node ((q / v) * 32 + l) * v + q % v of the
 // tile, v = 2 or 4 values of 8 or 4 bytes in a 16-byte vector, or 1.
 OGS_HD inline int lone_node(int l, int q, int v) { return ((q / v) * 32 + l) * v + q % v; }
+// Whether the v values from place `at` of a lone tile on lie in a field of N
+// nodes.  (begin + at + v passes 2^31 in the last tile of 2^31 - 1 nodes.)
+OGS_HD inline bool lone_vector_in(int32_t begin, int at, int v, int32_t N) { return at + v <= N - begin; }
 
 // Member of a wide tile's row: node | N member << 31, or none.
 constexpr uint32_t kNoWideId = 0xFFFFFFFFu;

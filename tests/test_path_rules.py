@@ -40,3 +40,13 @@ def test_scatter_in_node_order_takes_handles_with_most_nodes_in_rows(tmp_path):
     body = "ogs_handle_s h; h.N = 1000;\n"
     body += "".join(f"h.nnzT = {n}; out(scatter_share(&h));\n" for n in (1, 500, 749, 750, 1000))
     assert run(tmp_path, body) == [0, 0, 0, 1, 1]
+
+
+def test_lone_vectors_end_with_the_field(tmp_path):
+    """The last vectors of lone tiles, of the largest mesh too: none that reaches
+    past the last node is taken whole."""
+    cases = [(0, 0, 4, 4), (0, 0, 4, 3), (256, 252, 4, 512), (256, 252, 4, 511), (256, 254, 2, 511),
+             (2**31 - 256, 252, 4, 2**31 - 1), (2**31 - 256, 248, 4, 2**31 - 1), (2**31 - 256, 254, 2, 2**31 - 1),
+             (2**31 - 256, 254, 1, 2**31 - 1), (2**31 - 256, 255, 1, 2**31 - 1)]
+    got = run(tmp_path, "".join(f"out(lone_vector_in({b}, {at}, {v}, {n}));\n" for b, at, v, n in cases))
+    assert got == [int(b + at + v <= n) for b, at, v, n in cases]
