@@ -139,7 +139,8 @@ __device__ __forceinline__ bool lone_suspect(const T x) {
 template <typename T>
 __device__ __forceinline__ void lone_load_state(const DevMaps& m, const Tile& t, int lane, WarpState& s) {
   s.I[0] = t.begin;
-  s.emask = __ldg((sizeof(T) == 8 ? m.lmask8 : m.lmask4) + static_cast<int64_t>(t.count) * 32 + lane);
+  const uint32_t mask = __ldg((sizeof(T) == 8 ? m.lmask8 : m.lmask4) + static_cast<int64_t>(t.count) * 32 + lane);
+  s.emask = checked_lone_mask(mask, t.begin, lane, 16 / sizeof(T), m.b[1].nnodes, m.b[1].err);
 }
 
 template <typename T, int OP>

@@ -82,6 +82,26 @@ __device__ __forceinline__ int32_t checked_id(int32_t id, int32_t lim, unsigned 
   return id;
 }
 
+// A lane's byte of a lone tile's mask (vectors of v values), in checked builds
+// without the bits of nodes at and above `lim`, which are counted in *err.
+__device__ __forceinline__ uint32_t checked_lone_mask(uint32_t mask, int32_t begin, int lane, int v, int32_t lim,
+                                                      unsigned int* err) {
+#if OGS_CHECK_BOUNDS
+  for (int q = 0; q < 8; ++q)
+    if (((mask >> q) & 1u) && !lone_vector_in(begin, lone_node(lane, q, v), 1, lim)) {
+      if (err) atomicAdd(err, 1u);
+      mask &= ~(1u << q);
+    }
+#else
+  (void)begin;
+  (void)lane;
+  (void)v;
+  (void)lim;
+  (void)err;
+#endif
+  return mask;
+}
+
 template <typename T>
 __device__ __forceinline__ T type_max() {
   if constexpr (std::is_same<T, float>::value) return FLT_MAX;

@@ -165,13 +165,16 @@ __device__ __forceinline__ void warp_fold_store(const WarpState& s, T* dst, T* g
 // the tile, and a node's row follows from its word's first members.
 __device__ __forceinline__ void lone_rows(const DevMaps& m, const Tile& t, int lane, WarpState& s) {
   s.I[0] = t.begin;
-  s.emask = __ldg(m.lmask1 + static_cast<int64_t>(t.count) * 32 + lane);
+  const uint32_t mask = __ldg(m.lmask1 + static_cast<int64_t>(t.count) * 32 + lane);
+  s.emask = checked_lone_mask(mask, t.begin, lane, 1, m.b[1].nnodes, m.b[1].err);
   const NodeWord* w = m.nodes.words + (t.begin >> 5);
 #pragma unroll
   for (int q = 0; q < 8; ++q) {
     const uint2 f = __ldg(reinterpret_cast<const uint2*>(w + q));
     const int32_t row0 = __ldg(&w[q].row0);
-    s.R[q] = checked_id(row0 + __popc(f.x & ((1u << lane) - 1u)), m.b[1].nrows, m.b[1].err);
+    // (the sum is a row only for the lanes whose node is its row's first member)
+    if (!OGS_CHECK_BOUNDS || ((s.emask >> q) & 1u))
+      s.R[q] = checked_id(row0 + __popc(f.x & ((1u << lane) - 1u)), m.b[1].nrows, m.b[1].err);
   }
 }
 
