@@ -228,7 +228,12 @@ __device__ __forceinline__ void run_fixed(const DevBucket& b, const Tile& t, con
     }
   }
   const uint32_t gmask_on = pat.gather_n ? 1u : 0u;
-  const uint32_t smask_on = pat.scatter_n ? 1u : 0u;
+  uint32_t smask[RPT];  // the members that are written
+#pragma unroll
+  for (int j = 0; j < RPT; ++j) {
+    const uint32_t in_n = msk[j] & ((1u << D) - 1u);
+    smask[j] = !pat.scatter_n ? 0xFFu : (pat.scatter_n == 2 && !in_n ? 1u : in_n);
+  }
   const int K = K1 ? 1 : f.K;
   const int64_t stride = K1 ? 1 : (f.is_many ? 1 : K);
 
@@ -253,7 +258,13 @@ __device__ __forceinline__ void run_fixed(const DevBucket& b, const Tile& t, con
 #pragma unroll
       for (int j = 0; j < RPT; ++j) {
         T a;
-        if ((OP == OGS_ADD || OP == OGS_MUL) && !gmask_on) {
+        if (pat.gslib) {
+          // members are stored unflagged first, so member 0 takes part whenever any does
+          a = (!gmask_on || (msk[j] & 1u)) ? x[j][0] : op_init_gs<T, OP>();
+#pragma unroll
+          for (int m = 1; m < D; ++m)
+            if (!gmask_on || ((msk[j] >> m) & 1u)) op_apply<T, OP>(a, x[j][m]);
+        } else if ((OP == OGS_ADD || OP == OGS_MUL) && !gmask_on) {
           a = fold_from_first<T, OP, D>(x[j], 0);
         } else {
           a = op_init<T, OP>();
@@ -275,8 +286,7 @@ __device__ __forceinline__ void run_fixed(const DevBucket& b, const Tile& t, con
       for (int j = 0; j < RPT; ++j) {
 #pragma unroll
         for (int m = 0; m < D; ++m)
-          if (ok[j] && (!smask_on || ((msk[j] >> m) & 1u)))
-            dst[static_cast<int64_t>(c[j][m]) * stride] = val[j];
+          if (ok[j] && ((smask[j] >> m) & 1u)) dst[static_cast<int64_t>(c[j][m]) * stride] = val[j];
       }
     }
   }
