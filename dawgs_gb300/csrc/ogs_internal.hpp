@@ -254,6 +254,11 @@ struct FieldArgs {
   int32_t overlap = 0;      // host: launch with programmatic stream serialization
 };
 
+// Whether the pipelines and the wide tiles take a call of K components: they
+// number a tile's 32 K (row lane, component) units in 32 bits.  The direct kernel
+// (ogs_kernels.cuh) steps through components in 64.
+inline bool units_fit(int K, bool is_many) { return is_many || K <= (1 << 27); }
+
 // Whether a Scatter runs in node order (ogs_scatter.cuh): where the handle has
 // node words (rows numbered by first member) and most of its nodes take part
 // (scatter_share), for up to kScatterMaxK components.

@@ -179,7 +179,8 @@ __device__ __forceinline__ T* field_base(const FieldArgs& f, int k) {
   return f.is_many ? static_cast<T*>(f.many[k]) : static_cast<T*>(f.v) + k;
 }
 
-// Value `i` of a component, values a stride apart: in bytes below 2^32, a
+// Value `i` of a component, values a stride apart: in bytes below 2^32
+// (units_fit: at most 2^30), a
 // product and sum in one instruction instead of three (21x18x20 p=7 masked
 // Trans k=2 30.9 -> 26.9 us a call, 24^3 p=3 k=8 21.2 -> 18.6), or in values.
 struct ByteStride {

@@ -33,8 +33,7 @@ namespace ogsgb {
 
 template <typename T, int OP, int MODE>
 inline cudaError_t launch_mode(const DevMaps& m, const FieldArgs& f, Pattern pat, cudaStream_t s) {
-  // the pipelines step through components by a 32-bit number of bytes
-  if (!f.is_many && static_cast<uint64_t>(f.K) * sizeof(T) > 0xFFFFFFFFull) return launch_direct<T, OP, MODE>(m, f, pat, s);
+  if (!units_fit(f.K, f.is_many != 0)) return launch_direct<T, OP, MODE>(m, f, pat, s);
   if constexpr (OGS_KERNEL == 2) {
     return launch_direct<T, OP, MODE>(m, f, pat, s);
   } else if constexpr (OGS_ASYNC != 0) {

@@ -50,3 +50,13 @@ def test_lone_vectors_end_with_the_field(tmp_path):
              (2**31 - 256, 254, 1, 2**31 - 1), (2**31 - 256, 255, 1, 2**31 - 1)]
     got = run(tmp_path, "".join(f"out(lone_vector_in({b}, {at}, {v}, {n}));\n" for b, at, v, n in cases))
     assert got == [int(b + at + v <= n) for b, at, v, n in cases]
+
+
+def test_units_of_a_tile_fit_32_bits(tmp_path):
+    """The largest k that the pipelines and wide tiles take keeps its last unit and
+    its bytes below 2^32; separate arrays always do."""
+    got = run(tmp_path, "".join(f"out(units_fit({k}, false)); out(units_fit({k}, true));\n" for k in KS))
+    assert got[1::2] == [1] * len(KS)
+    for k, fit in zip(KS, got[::2]):
+        assert fit == int(32 * k - 1 < 2**32), k
+        assert not fit or 8 * k < 2**32
