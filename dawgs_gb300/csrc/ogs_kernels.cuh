@@ -51,8 +51,9 @@ enum KLayout : int {
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
 
+// (An error stays with the runtime, for the caller's cudaGetLastError.)
 template <typename... P, typename... A>
-inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t s,
+inline void launch_overlapped(void (*kernel)(P...), dim3 grid, int block, size_t smem, cudaStream_t s,
                                      bool overlap, A... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
@@ -64,7 +65,7 @@ inline cudaError_t launch_overlapped(void (*kernel)(P...), dim3 grid, int block,
   attr.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = overlap ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+  cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 
 // A column or row id loaded from the maps, checked against [0, lim) in

@@ -90,8 +90,9 @@ inline cudaError_t launch_scatter_as(const DevMaps& m, const FieldArgs& f, cudaS
   };
   const int block = ctas(kScatterBlock) < kScatterCtas ? kScatterSmallBlock : kScatterBlock;
   const dim3 grid(static_cast<unsigned>(ctas(block)));
-  return launch_overlapped(ogs_scatter_kernel<T, K, NONLY>, grid, block, 0, s, f.overlap, m.nodes,
-                           static_cast<T*>(f.v), static_cast<const T*>(f.gv), m.b[1].nrows, m.b[1].err);
+  launch_overlapped(ogs_scatter_kernel<T, K, NONLY>, grid, block, 0, s, f.overlap, m.nodes, static_cast<T*>(f.v),
+                    static_cast<const T*>(f.gv), m.b[1].nrows, m.b[1].err);
+  return cudaGetLastError();
 }
 
 template <typename T, bool NONLY>
