@@ -21,6 +21,7 @@ SETUP_VERBOSE = 1
 SETUP_HOST_ONLY = 2
 SETUP_DEVICE_MAPS = 4
 SETUP_HOST_MAPS = 8
+SETUP_NO_OVERLAP = 16
 DEVICE_MAPS_MIN_N = 65536
 
 # every symbol include/ogs_c.h declares: (name, restype, argtypes)

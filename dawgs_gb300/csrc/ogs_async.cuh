@@ -228,9 +228,8 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_async_kernel(const 
   // ahead (grid_wait).  With components the wait in the middle costs more
   // registers than it hides: 32x32x16 p=5 permuted k=3 fp32 27.3 us a call
   // against 26.4 with the wait up here, Gather 23.0 against 18.6.
-  grid_release();
   constexpr bool kLate = PLAIN && KL == kK1;
-  if (!kLate || i0 >= nitems) grid_wait();
+  if (!kLate || i0 >= nitems) grid_wait(f.overlap);
   if (i0 >= nitems) return;
   int64_t i = i0;
   const int64_t step = W, iend = nitems;
@@ -311,7 +310,7 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_async_kernel(const 
     else OGS_DEGREE_SWITCH(nxt.bucket, OGS_A_LOAD_NXT)
 #undef OGS_A_LOAD_NXT
   }
-  if (kLate) grid_wait();  // the first access to the field follows
+  if (kLate) grid_wait(f.overlap);  // the first access to the field follows
   {
     const T* src = (MODE == kModeScatter) ? nullptr : field_base<T>(f, kcur);
 #define OGS_A_ISSUE0(D) async_issue_vals<T, MODE, D>(scur, src, gv, stride, K, kcur, gmask, rcur, lane, ring)

@@ -104,7 +104,7 @@ ogs_status launch(const ogs_handle_s* h, const FieldArgs& f, int mode, int op, P
 // persistent CTAs of the next call's other need (gs of 32x32x24 cells of six p=3
 // tetrahedra: copy and four calls 151 us overlapped, 128 not).
 int may_overlap(const ogs_handle_s* h, void* stream) {
-  if (h->dmaps.ngtiles > 0) return 0;
+  if (!h->overlap || h->dmaps.ngtiles > 0) return 0;
   cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &c) != cudaSuccess) {
     cudaGetLastError();
@@ -269,6 +269,7 @@ ogs_status ogs_setup_ex(ogs_handle* out, int64_t N, int64_t* ids, int kind, int 
                                : build_host_maps(h, N, ids, kind, unique);
     if (s != OGS_OK) { release_device(h); delete h; return s; }
     h->host_only = host_only;
+    h->overlap = !(flags & OGS_SETUP_NO_OVERLAP);
     if (!h->arena) build_layout(h);  // the device path built it already (unless the maps are empty)
     if (!h->host_only && !h->arena) {
       s = upload_layout(h);

@@ -197,7 +197,9 @@ constexpr int kLoneBucket = kDmax + 1;
 OGS_HD inline int lone_node(int l, int q, int v) { return ((q / v) * 32 + l) * v + q % v; }
 // Whether the v values from place `at` of a lone tile on lie in a field of N
 // nodes.  (begin + at + v passes 2^31 in the last tile of 2^31 - 1 nodes.)
-OGS_HD inline bool lone_vector_in(int32_t begin, int at, int v, int32_t N) { return at + v <= N - begin; }
+OGS_HD inline bool lone_vector_in(int32_t begin, int at, int v, int32_t N) {
+  return static_cast<uint32_t>(begin) + static_cast<uint32_t>(at + v) <= static_cast<uint32_t>(N);
+}
 
 // Member of a wide tile's row: node | N member << 31, or none.
 constexpr uint32_t kNoWideId = 0xFFFFFFFFu;
@@ -251,7 +253,7 @@ struct FieldArgs {
   void* many[kMaxMany];     // separate arrays (GS many)
   int32_t K;
   int32_t is_many;
-  int32_t overlap = 0;      // host: launch with programmatic stream serialization
+  int32_t overlap = 0;      // programmatic stream serialization (grid_wait)
 };
 
 // Whether the pipelines and the wide tiles take a call of K components: they
@@ -329,6 +331,7 @@ struct ogs_handle_s {
   bool covers_all = false;  // every local node is in the T map (no zero ids)
   bool gslib = false;       // maps in gslib's member order (ogs_gslib.cpp)
   bool from_maps = false;   // an operator over caller-built maps (ogs_maps.cpp)
+  bool overlap = true;      // calls may start before the work ahead of them has ended
   bool distinct_cols = true;  // no local node in two rows (GatherScatter/Scatter need it)
 
   std::vector<int32_t> rowStartsT, colIdsT, rowStartsN, colIdsN;  // N empty when Unsigned

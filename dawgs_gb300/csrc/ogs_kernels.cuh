@@ -40,16 +40,24 @@ enum KLayout : int {
                     // the grid sweeps that array
 };
 
-// Programmatic dependent launch.  A call's kernels let the next one in the
-// stream start as their CTAs leave (grid_release) and, before they touch a
-// field, wait for the work before them (grid_wait: whole grids, their writes
-// visible); until then they read maps only, which do not change after setup.
-// Both are nothing for kernels launched without the attribute.  It hides the
-// gap between launches and the first two of a call's three chained loads: 24^3
+// Programmatic dependent launch (FieldArgs::overlap).  A call's kernel may start
+// before the work ahead of it in the stream has ended; before it touches a field
+// it waits for that work (whole grids, their writes visible), and until then it
+// reads maps only, which do not change after setup.  With `release` it lets the
+// next kernel start from there on, not earlier: what that one runs before its own
+// wait, a kernel of another library's too, finds everything ahead of this call
+// done.  Kernels launched without overlap release nothing.  It hides the gap
+// between launches and the first two of a call's three chained loads: 24^3
 // p=7 fp64 copy and four GatherScatters 116.5 -> 109.0 us, Scatter then Gather
-// 49.8 -> 43.4, 23x19x17 p=6 int64 copy and Max 24.6 -> 22.3.
-__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
-__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+// 49.8 -> 43.4, 23x19x17 p=6 int64 copy and Max 24.6 -> 22.3.  (Released at the
+// top of the kernel: the same within 0.1 us a call.  The predicate in one asm
+// block, since a branch around the release cost 24^3 p=15 0.6 %.)
+__device__ __forceinline__ void grid_wait(int release) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.s32 p, %0, 0;\n griddepcontrol.wait;\n @p griddepcontrol.launch_dependents;\n}\n" ::"r"(
+          release)
+      : "memory");
+}
 
 // (An error stays with the runtime, for the caller's cudaGetLastError.)
 template <typename... P, typename... A>

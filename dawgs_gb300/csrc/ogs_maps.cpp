@@ -108,6 +108,7 @@ extern "C" ogs_status ogs_setup_maps(ogs_handle* out, int64_t N, int64_t NrowsN,
     }
     build_layout(h);
     h->host_only = (flags & OGS_SETUP_HOST_ONLY) != 0;
+    h->overlap = !(flags & OGS_SETUP_NO_OVERLAP);
     if (!h->host_only) {
       s = upload_layout(h);
       if (s != OGS_OK) { release_device(h); delete h; return s; }

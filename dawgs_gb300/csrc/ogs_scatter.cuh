@@ -42,13 +42,13 @@ OGS_HD constexpr int scatter_words(int K) { return K == 1 ? 8 : K == 2 ? 4 : K <
 // their nodes from the other lanes.  NONLY: writes N members only (Trans).
 template <typename T, int K, bool NONLY>
 __global__ void __launch_bounds__(kScatterBlock) ogs_scatter_kernel(const DevNodes m, T* v, const T* gv,
-                                                                    const int32_t nrows, unsigned int* err) {
+                                                                    const int32_t nrows, unsigned int* err,
+                                                                    const int release) {
   constexpr int W = scatter_words(K);
   const int lane = static_cast<int>(threadIdx.x) & 31;
   const int64_t w0 = (static_cast<int64_t>(blockIdx.x) * (blockDim.x / 32) + (threadIdx.x >> 5)) * W;
-  grid_release();
   if (w0 >= m.nwords) {
-    grid_wait();
+    grid_wait(release);
     return;
   }
   NodeWord w[W];
@@ -64,7 +64,7 @@ __global__ void __launch_bounds__(kScatterBlock) ogs_scatter_kernel(const DevNod
     if (r[j] >= 0) r[j] = checked_id(r[j], nrows, err);
     if (NONLY && !((m.nmem[w0 + j] >> lane) & 1u)) r[j] = -1;
   }
-  grid_wait();
+  grid_wait(release);
   T x[W][K];
   int32_t row[W][K];
 #pragma unroll
@@ -91,7 +91,7 @@ inline cudaError_t launch_scatter_as(const DevMaps& m, const FieldArgs& f, cudaS
   const int block = ctas(kScatterBlock) < kScatterCtas ? kScatterSmallBlock : kScatterBlock;
   const dim3 grid(static_cast<unsigned>(ctas(block)));
   launch_overlapped(ogs_scatter_kernel<T, K, NONLY>, grid, block, 0, s, f.overlap, m.nodes, static_cast<T*>(f.v),
-                    static_cast<const T*>(f.gv), m.b[1].nrows, m.b[1].err);
+                    static_cast<const T*>(f.gv), m.b[1].nrows, m.b[1].err, f.overlap);
   return cudaGetLastError();
 }
 

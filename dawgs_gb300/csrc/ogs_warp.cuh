@@ -212,9 +212,8 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_warp_kernel(const D
   const int nw = m.nwtiles;
   const int64_t i0 = static_cast<int64_t>(blockIdx.x) * (kBlock / 32) + (threadIdx.x >> 5);
   const bool idle = i0 >= static_cast<int64_t>(nw) * K;
-  grid_release();
   constexpr bool kLate = PLAIN && KL == kK1;
-  if (!kLate || idle) grid_wait();
+  if (!kLate || idle) grid_wait(f.overlap);
   if (idle) return;
   const bool use_mask = !PLAIN && (pat.gather_n || pat.scatter_n) && m.signed_maps;
   const bool gmask = !PLAIN && pat.gather_n != 0;
@@ -269,7 +268,7 @@ __global__ void __launch_bounds__(kBlock, OGS_WARP_MINB) ogs_warp_kernel(const D
   if (KL == kK1 ? i + W < nitems : ahead) nxt = m.wtiles[pnxt.t];
 
   T* gv = static_cast<T*>(f.gv);
-  if (kLate) grid_wait();  // (as in ogs_async.cuh)
+  if (kLate) grid_wait(f.overlap);  // (as in ogs_async.cuh)
   for (;;) {
     const int k0 = ccur;
     const T* src = (MODE == kModeScatter) ? nullptr : field_base<T>(f, k0);

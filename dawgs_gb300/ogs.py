@@ -155,9 +155,11 @@ class ogs_t:
 
     # ogs_t::Setup, include/ogs.hpp:221-228 / libs/ogs/ogsSetup.cpp:44-53
     def Setup(self, N, ids, comm=None, kind=Unsigned, method=Auto, unique=False,
-              verbose=False, platform=None, host_only=False, maps=None):
+              verbose=False, platform=None, host_only=False, maps=None, overlap=True):
         """maps: None (GPU for N >= 65536 unless host_only), "device" or "host"
-        -- where the N/T maps are built; the handle is the same either way."""
+        -- where the N/T maps are built; the handle is the same either way.
+        overlap=False: device calls start only when the work ahead of them has
+        ended (OGS_SETUP_NO_OVERLAP)."""
         self.Free()
         if not (isinstance(ids, np.ndarray) and ids.dtype == np.int64 and ids.flags.c_contiguous):
             raise OgsError(_lib.OGS_EINVAL, "ids must be a contiguous int64 numpy array")
@@ -165,6 +167,7 @@ class ogs_t:
             raise OgsError(_lib.OGS_EINVAL, "ids is shorter than N")
         h = C.c_void_p()
         flags = (_lib.SETUP_VERBOSE if verbose else 0) | (_lib.SETUP_HOST_ONLY if host_only else 0)
+        flags |= 0 if overlap else _lib.SETUP_NO_OVERLAP
         if maps not in (None, "device", "host"):
             raise OgsError(_lib.OGS_EINVAL, "maps must be None, 'device' or 'host'")
         flags |= {None: 0, "device": _lib.SETUP_DEVICE_MAPS, "host": _lib.SETUP_HOST_MAPS}[maps]

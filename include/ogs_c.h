@@ -16,7 +16,14 @@
  *
  * Operations are asynchronous on `stream` unless the name ends in _host.  A
  * handle's maps are immutable after setup, so device-buffer calls on one
- * handle from several streams and threads are safe.  The _host calls share
+ * handle from several streams and threads are safe.  Outside a stream capture,
+ * a device call's kernel may be scheduled before the work ahead of it in the
+ * stream has ended; it touches no field until that work is done and visible.
+ * In turn it lets a kernel behind it start early if that kernel was launched with
+ * programmatic stream serialization (nothing else is affected): such a kernel's
+ * part before its own wait (griddepcontrol.wait, cudaGridDependencySynchronize)
+ * may run while the call does, and finds everything ahead of the call done.
+ * OGS_SETUP_NO_OVERLAP turns both off for a handle.  The _host calls share
  * the handle's device staging buffer: a lock in the handle serialises them
  * (each returns only after its stream has synchronised), and they allocate
  * that buffer on first use unless ogs_reserve_host made it at setup time.
@@ -63,6 +70,9 @@ typedef enum { OGS_UNSIGNED = 0, OGS_SIGNED = 1, OGS_HALO = 2 } ogs_kind;
 #define OGS_SETUP_DEVICE_MAPS 4u /* sort and scan on the GPU; not with HOST_ONLY */
 #define OGS_SETUP_HOST_MAPS   8u /* hash-table pass on the host */
 #define OGS_DEVICE_MAPS_MIN_N 65536
+/* The handle's calls start only when the work ahead of them has ended, and let
+ * no kernel start before they have (see "Operations are asynchronous" above). */
+#define OGS_SETUP_NO_OVERLAP  16u
 
 typedef struct {
   int64_t N;              /* local nodes (ogsBase_t::N) */
@@ -196,7 +206,7 @@ ogs_status ogs_checked_id_errors(ogs_handle h, uint64_t *count);
  * refused when a local node sits in two rows.  ogs_gather may run in place
  * (d_gv == d_v) when no row reads an entry another row's result overwrites:
  * postmpi's maps (row n = own entry n, then received entries) are such.
- * flags: OGS_SETUP_HOST_ONLY or 0. */
+ * flags: OGS_SETUP_HOST_ONLY, OGS_SETUP_NO_OVERLAP or 0. */
 ogs_status ogs_setup_maps(ogs_handle *out, int64_t N, int64_t NrowsN, int64_t NrowsT,
                           const int32_t *rowStartsN, const int32_t *colIdsN,
                           const int32_t *rowStartsT, const int32_t *colIdsT, unsigned flags);
@@ -246,7 +256,7 @@ ogs_status ogs_halo_setup(ogs_halo *out, int64_t N, const int64_t *ids, int meth
 /* A halo over the gatherHalo maps that the reference's multi-rank setup
  * builds (ogsSetup.cpp:569-776: NhaloP rows with an N member first, NhaloT rows
  * in all; N maps may be NULL for Unsigned), as in ogs_setup_maps; Nrecv rows of
- * extra buffer for the exchange.  flags: OGS_SETUP_HOST_ONLY or 0. */
+ * extra buffer for the exchange.  flags: as in ogs_setup_maps. */
 ogs_status ogs_halo_setup_maps(ogs_halo *out, int64_t N, int64_t NhaloP, int64_t NhaloT,
                                const int32_t *rowStartsN, const int32_t *colIdsN,
                                const int32_t *rowStartsT, const int32_t *colIdsT, int64_t Nrecv,
