@@ -40,13 +40,12 @@ OGS_HD constexpr int scatter_words(int K) { return K == 1 ? 8 : K == 2 ? 4 : K <
 // The 32 nodes of a word hold 32 K consecutive values: a lane first finds the
 // row of one node, then writes values lane, lane + 32, ... with the rows of
 // their nodes from the other lanes.  NONLY: writes N members only (Trans).
-template <typename T, int K, bool NONLY>
-__global__ void __launch_bounds__(kScatterBlock) ogs_scatter_kernel(const DevNodes m, T* v, const T* gv,
-                                                                    const int32_t nrows, unsigned int* err,
-                                                                    const int release) {
+template <typename T, int K, bool NONLY, int BLOCK>
+__global__ void __launch_bounds__(BLOCK) ogs_scatter_kernel(const DevNodes m, T* v, const T* gv, const int32_t nrows,
+                                                            unsigned int* err, const int release) {
   constexpr int W = scatter_words(K);
   const int lane = static_cast<int>(threadIdx.x) & 31;
-  const int64_t w0 = (static_cast<int64_t>(blockIdx.x) * (blockDim.x / 32) + (threadIdx.x >> 5)) * W;
+  const int64_t w0 = (static_cast<int64_t>(blockIdx.x) * (BLOCK / 32) + (threadIdx.x >> 5)) * W;
   if (w0 >= m.nwords) {
     grid_wait(release);
     return;
@@ -71,9 +70,10 @@ __global__ void __launch_bounds__(kScatterBlock) ogs_scatter_kernel(const DevNod
   for (int j = 0; j < W; ++j)
 #pragma unroll
     for (int q = 0; q < K; ++q) {
-      const int u = q * 32 + lane;
-      row[j][q] = K == 1 ? r[j] : __shfl_sync(0xffffffffu, r[j], u / K);
-      if (row[j][q] >= 0) x[j][q] = gv[static_cast<int64_t>(row[j][q]) * K + u % K];
+      const uint32_t u = static_cast<uint32_t>(q * 32 + lane);
+      const uint32_t n = u / K;
+      row[j][q] = K == 1 ? r[j] : __shfl_sync(0xffffffffu, r[j], n & 31);
+      if (row[j][q] >= 0) x[j][q] = gv[static_cast<int64_t>(row[j][q]) * K + (u - n * K)];
     }
 #pragma unroll
   for (int j = 0; j < W; ++j)
@@ -82,17 +82,25 @@ __global__ void __launch_bounds__(kScatterBlock) ogs_scatter_kernel(const DevNod
       if (row[j][q] >= 0) v[(w0 + j) * 32 * K + q * 32 + lane] = x[j][q];
 }
 
-template <typename T, int K, bool NONLY>
-inline cudaError_t launch_scatter_as(const DevMaps& m, const FieldArgs& f, cudaStream_t s) {
-  auto ctas = [&](int block) {
-    const int64_t per_block = scatter_words(K) * (block / 32);
-    return (m.nodes.nwords + per_block - 1) / per_block;
-  };
-  const int block = ctas(kScatterBlock) < kScatterCtas ? kScatterSmallBlock : kScatterBlock;
-  const dim3 grid(static_cast<unsigned>(ctas(block)));
-  launch_overlapped(ogs_scatter_kernel<T, K, NONLY>, grid, block, 0, s, f.overlap, m.nodes, static_cast<T*>(f.v),
+template <int K>
+inline int64_t scatter_ctas(int64_t nwords, int block) {
+  const int64_t per_block = scatter_words(K) * (block / 32);
+  return (nwords + per_block - 1) / per_block;
+}
+
+template <typename T, int K, bool NONLY, int BLOCK>
+inline cudaError_t launch_scatter_block(const DevMaps& m, const FieldArgs& f, cudaStream_t s) {
+  const dim3 grid(static_cast<unsigned>(scatter_ctas<K>(m.nodes.nwords, BLOCK)));
+  launch_overlapped(ogs_scatter_kernel<T, K, NONLY, BLOCK>, grid, BLOCK, 0, s, f.overlap, m.nodes, static_cast<T*>(f.v),
                     static_cast<const T*>(f.gv), m.b[1].nrows, m.b[1].err, f.overlap);
   return cudaGetLastError();
+}
+
+template <typename T, int K, bool NONLY>
+inline cudaError_t launch_scatter_as(const DevMaps& m, const FieldArgs& f, cudaStream_t s) {
+  if (scatter_ctas<K>(m.nodes.nwords, kScatterBlock) < kScatterCtas)
+    return launch_scatter_block<T, K, NONLY, kScatterSmallBlock>(m, f, s);
+  return launch_scatter_block<T, K, NONLY, kScatterBlock>(m, f, s);
 }
 
 template <typename T, bool NONLY>
