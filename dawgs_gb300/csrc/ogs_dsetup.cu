@@ -860,6 +860,7 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
   m.wide = d_wide;
   m.wide_ids = d_wids;
   m.nwide = static_cast<int32_t>(nwide);
+  m.wide_short = L.g_nnzT <= 12 * L.g_n;
   m.nodes.words = d_words;
   m.nodes.nmem = reinterpret_cast<const uint32_t*>(base + o_nmem);
   m.nodes.orow = reinterpret_cast<const int32_t*>(base + o_orow);

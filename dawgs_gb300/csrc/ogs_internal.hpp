@@ -224,6 +224,7 @@ struct DevMaps {
   const Tile* wide;
   const uint32_t* wide_ids;
   int32_t nwide;           // 0: the general rows run as CTA tiles
+  int32_t wide_short;      // the rows are of degree 12 and less on average
   // The warp tiles of degree 2 and up with lone tiles in place of the degree-1
   // ones, in node order, for handles that are mostly lone nodes (wants_lone).
   const Tile* ltiles;

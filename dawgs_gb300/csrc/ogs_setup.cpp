@@ -696,6 +696,7 @@ ogs_status upload_layout(ogs_handle_s* h) {
   m.wide = reinterpret_cast<const Tile*>(base + o_wide);
   m.wide_ids = reinterpret_cast<const uint32_t*>(base + o_wids);
   m.nwide = static_cast<int32_t>(L.wide.size());
+  m.wide_short = L.g_nnzT <= 12 * L.g_n;
   m.nodes.words = reinterpret_cast<const NodeWord*>(base + o_words);
   m.nodes.nmem = reinterpret_cast<const uint32_t*>(base + o_nmem);
   m.nodes.orow = reinterpret_cast<const int32_t*>(base + o_orow);
