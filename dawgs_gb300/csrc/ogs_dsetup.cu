@@ -25,7 +25,7 @@
 // ogs_get_maps.  Both paths give identical handles.
 //
 // Every buffer here is scratch of the setup call and is freed before it
-// returns.  Device memory needed: 78 bytes per local node (91 Signed).
+// returns.  Device memory needed: 78 bytes per local node (87 Signed) and 8 MB.
 #include <algorithm>
 #include <cstdint>
 #include <limits>
@@ -507,8 +507,10 @@ __global__ void k_node_others(const int32_t* __restrict__ code, const int32_t* _
 // from a mark on can be given up for others once the work that uses them is
 // queued: all of it runs on one stream.  Meshes below kBlockNodes do without the
 // block: their pieces fit what the driver holds already, and the block, at least
-// 8 MB, does not (setup, block / pieces: 512 nodes 477 / 401 us, 4,096 499 / 436,
-// 32,768 549 / 606, 216,000 602 / 1,248, 7,077,888 2.90 / 4.16 ms).
+// 8 MB, does not.  Setup, block / pieces, us, Unsigned and Signed unique: 4,096
+// nodes 498 / 438 and 584 / 533, 16,384 539 / 477 and 625 / 578, 24,576 537 / 478
+// and 623 / 723, 32,768 545 / 609 and 632 / 719, 65,536 569 / 714 and 661 / 820,
+// 131,072 607 / 989 and 715 / 1,168.
 constexpr int64_t kBlockNodes = 32768;
 
 struct Scratch {

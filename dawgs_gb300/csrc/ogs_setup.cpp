@@ -22,6 +22,7 @@
 #include <cstring>
 #include <climits>
 #include <limits>
+#include <memory>
 
 #include <cuda_runtime.h>
 
@@ -355,26 +356,31 @@ void build_layout(ogs_handle_s* h) {
   L.nmem.clear();
   L.orow.clear();
   if (wants_node_words(h)) {
-    std::vector<int32_t> rowof(static_cast<size_t>(h->N), -1);
+    // Rows ascend with their first members, so the first one met in a word gives
+    // its row0; the other members' rows wait at their nodes for the words' order.
+    // (Node by node, each looking at its row's first member, took 2 to 4 % longer
+    // in Setup of Signed unique meshes below 65,536 nodes.)
+    const std::unique_ptr<int32_t[]> rowof(new int32_t[static_cast<size_t>(h->N)]);
     L.nwords.assign(node_words_padded(h->N), NodeWord{0, 0, 0, 0});
     L.nmem.assign(L.nwords.size(), 0);
     for (int64_t r = 0; r < R; ++r) {
-      for (int32_t q = rsT[r]; q < rsT[r + 1]; ++q) rowof[ciT[q]] = static_cast<int32_t>(r);
+      const int32_t first = ciT[rsT[r]];
+      NodeWord& w = L.nwords[first >> 5];
+      if (!w.first) w.row0 = static_cast<int32_t>(r);
+      w.first |= 1u << (first & 31);
+      for (int32_t q = rsT[r] + 1; q < rsT[r + 1]; ++q) {
+        const int32_t c = ciT[q];
+        L.nwords[c >> 5].other |= 1u << (c & 31);
+        rowof[c] = static_cast<int32_t>(r);
+      }
       for (int32_t q = rsN[r]; q < rsN[r + 1]; ++q) L.nmem[ciN[q] >> 5] |= 1u << (ciN[q] & 31);
     }
-    L.orow.reserve(h->nnzT - R);
-    for (int64_t n = 0; n < h->N; ++n) {
-      NodeWord& w = L.nwords[n >> 5];
-      const int32_t r = rowof[n];
-      if ((n & 31) == 0) w.other0 = static_cast<int32_t>(L.orow.size());
-      if (r < 0) continue;
-      if (ciT[rsT[r]] == n) {
-        if (!w.first) w.row0 = r;
-        w.first |= 1u << (n & 31);
-      } else {
-        w.other |= 1u << (n & 31);
-        L.orow.push_back(r);
-      }
+    L.orow.resize(static_cast<size_t>(h->nnzT - R));
+    int32_t* to = L.orow.data();
+    for (int64_t i = 0; i < node_words(h->N); ++i) {
+      NodeWord& w = L.nwords[i];
+      w.other0 = static_cast<int32_t>(to - L.orow.data());
+      for (uint32_t rest = w.other; rest; rest &= rest - 1) *to++ = rowof[i * 32 + __builtin_ctz(rest)];
     }
   }
   L.g_n = static_cast<int64_t>(L.g_rows.size());
@@ -632,6 +638,12 @@ ogs_status upload_layout(ogs_handle_s* h) {
   const uint32_t zero = 0;
   const size_t o_err = add(&zero, sizeof(zero));  // ids out of range (checked builds)
 
+  // Neighbouring small pieces go in one copy: a copy costs 6 us whatever its size,
+  // and the three of the words made Setup of 512 Signed unique nodes 269 -> 291 us
+  // (now 134), of 64,000 2,102 -> 2,286 (2,084).
+  constexpr size_t kSmallPiece = 64 << 10, kRun = 1 << 20;
+  std::vector<char> run;
+  run.reserve(std::min(total, kRun));
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return set_error(OGS_EDEVICE, std::string("cudaGetDevice: ") + cudaGetErrorString(e));
@@ -652,13 +664,29 @@ ogs_status upload_layout(ogs_handle_s* h) {
     r.stride = static_cast<int32_t>(L.rows[w.bucket].size());
     r.nP = L.nP[w.bucket];
   }
+  size_t run_off = 0;
+  auto copy = [&](size_t off, const void* src, size_t bytes) {
+    if (e == cudaSuccess && bytes) e = cudaMemcpy(base + off, src, bytes, cudaMemcpyHostToDevice);
+  };
+  auto flush = [&] {
+    copy(run_off, run.data(), run.size());
+    run.clear();
+  };
   for (const Piece& p : pieces) {
     if (!p.bytes) continue;
-    e = cudaMemcpy(base + p.off, p.src, p.bytes, cudaMemcpyHostToDevice);
-    if (e != cudaSuccess) {
-      dev_free(base);
-      return set_error(OGS_EDEVICE, std::string("cudaMemcpy of maps: ") + cudaGetErrorString(e));
+    if (p.bytes > kSmallPiece || (!run.empty() && p.off + p.bytes - run_off > kRun)) flush();
+    if (p.bytes > kSmallPiece) {
+      copy(p.off, p.src, p.bytes);
+      continue;
     }
+    if (run.empty()) run_off = p.off;
+    run.resize(p.off - run_off);  // (the pieces' alignment)
+    run.insert(run.end(), static_cast<const char*>(p.src), static_cast<const char*>(p.src) + p.bytes);
+  }
+  flush();
+  if (e != cudaSuccess) {
+    dev_free(base);
+    return set_error(OGS_EDEVICE, std::string("cudaMemcpy of maps: ") + cudaGetErrorString(e));
   }
   h->device = dev;
   h->arena = base;
