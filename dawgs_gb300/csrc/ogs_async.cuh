@@ -419,7 +419,8 @@ template <typename T, int OP, int MODE, int KL>
 inline void launch_async_kl(const DevMaps& m, const FieldArgs& f, Pattern pat, cudaStream_t s) {
   const bool plain = !pat.gather_n && !pat.scatter_n && !pat.limit_n && !pat.gslib;
   if constexpr (MODE == kModeGS && KL != kKInterleaved) {
-    bool lone = plain && m.nltiles > 0;
+    constexpr bool cheap = OP == OGS_MAX || OP == OGS_MIN || lone_is_noop<T, OP>();
+    bool lone = plain && lone_folds(m, sizeof(T), cheap);
     for (int k = 0; lone && k < (KL == kKMany ? f.K : 1); ++k)
       lone = (reinterpret_cast<uintptr_t>(KL == kKMany ? f.many[k] : f.v) & 15) == 0;
     if (lone) {

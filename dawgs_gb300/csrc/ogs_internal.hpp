@@ -262,6 +262,28 @@ struct FieldArgs {
 // (ogs_kernels.cuh) steps through components in 64.
 inline bool units_fit(int K, bool is_many) { return is_many || K <= (1 << 27); }
 
+// Whether a plain GatherScatter of values of `bytes` bytes runs over the lone
+// tiles, and a plain Gather: from kLoneBytes a field on, where the column ids and
+// gathers that they save come out of DRAM, a quarter of L2 with the ids beside.
+// Below, a GatherScatter does from 65 % lone nodes on, or where the fold of a lone
+// node is the dearest (8-byte Max and Min of floats, a compare of 16 cycles) or
+// nothing (integers and Mul: `cheap`).  Us a call without / with them, Add: fp64
+// p=10 (55 %) 12^3 7.0 / 7.2, 14^3 (29 MB) 9.9 / 10.8, 16^3 (44 MB) 16.4 / 15.7,
+// 20^3 34.8 / 31.8; p=15 (67 %) 8^3 6.9 / 6.7, 12^3 (57 MB) 20.3 / 18.4; fp32 p=10
+// 14^3 7.9 / 8.8, 20^3 (43 MB) 26.4 / 22.7, p=13 (63 %) 12^3 (19 MB) 9.0 / 9.6,
+// 16^3 (45 MB) 25.2 / 21.5; four arrays of fp64 p=10 10^3 14.2 / 15.5, 24^3 243.7 /
+// 226.4.  Max fp64 p=10 10^3 6.1 / 5.3.  Gather fp64 p=10 14^3 9.3 / 10.1, 16^3
+// 15.8 / 13.6, p=15 8^3 6.6 / 6.9, fp32 p=10 16^3 (22 MB) 9.6 / 10.6, 20^3 26.5 /
+// 22.5.
+constexpr int64_t kLoneBytes = 30 << 20;
+inline bool lone_folds(const DevMaps& m, int bytes, bool cheap) {
+  const int64_t N = m.b[1].nnodes;
+  return m.nltiles > 0 && (N * bytes >= kLoneBytes || int64_t{20} * m.b[1].n >= 13 * N || (cheap && bytes == 8));
+}
+inline bool lone_gathers(const DevMaps& m, int bytes) {
+  return m.nltiles > 0 && m.nodes.nwords > 0 && int64_t{m.b[1].nnodes} * bytes >= kLoneBytes;
+}
+
 // Whether a Scatter runs in node order (ogs_scatter.cuh): where the handle has
 // node words (rows numbered by first member) and most of its nodes take part
 // (scatter_share), for up to kScatterMaxK components.
@@ -386,12 +408,13 @@ inline bool scatter_share(const ogs_handle_s* h) { return h->nnzT * 4 >= h->N * 
 // padding would outweigh the rows.
 int64_t wide_layout(const int32_t* starts, int64_t rows, std::vector<Tile>& wide);
 // Whether a handle gets lone tiles for its n1 rows of degree 1 (the rows being
-// numbered by first member): from 55 % of its nodes on.  Us a call without and
-// with them, boxes of 24^3: fp64 p=9 (51 %) 47.7 and 49.0, p=10 (55 %) 60.0 and
-// 60.2, p=11 (58 %) 76.4 and 75.4, p=15 (67 %) 185.7 and 158.0; fp32 p=11 60.2
-// and 56.5, p=7 (42 %) 17.5 and 19.1.  Gather fp64 p=7 25.1 and 24.6, p=9 46.6
-// and 44.5, p=11 77.8 and 72.2, p=15 189.4 and 162.3; fp32 p=7 13.3 and 14.8,
-// p=11 55.8 and 54.8.
+// numbered by first member): from 55 % of its nodes on; which calls run over them
+// is up to lone_folds and lone_gathers.  Us a call without and with them, boxes of
+// 24^3: GatherScatter fp64 p=9 (51 %) 47.7 and 49.0, p=10 (55 %) 58.2 and 58.5,
+// four arrays 243.7 and 226.4, p=11 (58 %) 75.2 and 74.3, p=15 (67 %) 185.1 and
+// 157.1; fp32 p=7 (42 %) 17.5 and 19.1, p=11 59.1 and 56.5, p=15 134.8 and 108.8.
+// Gather fp64 p=7 25.1 and 24.6, p=9 46.6 and 44.5, p=11 77.2 and 71.7, p=15 187.6
+// and 161.5; fp32 p=7 13.3 and 14.8, p=11 54.9 and 53.8.
 inline bool wants_lone(const ogs_handle_s* h, int64_t n1) {
   return !h->gslib && !h->from_maps && h->NlocalP == h->NlocalT && n1 * 20 >= h->N * 11;
 }

@@ -339,7 +339,7 @@ inline void launch_warp_kl(const DevMaps& m, const FieldArgs& f, Pattern pat, cu
 template <typename T, int OP, int MODE, bool PLAIN>
 inline void launch_warp_plain(const DevMaps& m, const FieldArgs& f, Pattern pat, cudaStream_t s) {
   if constexpr (MODE == kModeGather && PLAIN) {
-    if (f.K == 1 && m.nltiles > 0 && m.nodes.nwords > 0) {
+    if (f.K == 1 && lone_gathers(m, sizeof(T))) {
       DevMaps l = m;
       l.wtiles = m.ltiles;
       l.nwtiles = m.nltiles;

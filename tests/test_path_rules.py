@@ -60,3 +60,19 @@ def test_units_of_a_tile_fit_32_bits(tmp_path):
     for k, fit in zip(KS, got[::2]):
         assert fit == int(32 * k - 1 < 2**32), k
         assert not fit or 8 * k < 2**32
+
+
+def test_lone_tiles_by_the_field_and_the_share(tmp_path):
+    """Handles with lone tiles: large fields, mostly lone nodes, and 8-byte folds
+    that cost more or nothing."""
+    body = "DevMaps m{}; m.nltiles = 3; m.nodes.nwords = 9;\n"
+    cases = [(n, lone, b, c) for n in (1000, 4000000, 8000000) for lone in (0.56, 0.66) for b in (4, 8) for c in (0, 1)]
+    for n, lone, b, c in cases:
+        body += f"m.b[1].nnodes = {n}; m.b[1].n = {int(n * lone)}; out(lone_folds(m, {b}, {c})); out(lone_gathers(m, {b}));\n"
+    body += "m.nodes.nwords = 0; out(lone_gathers(m, 8)); m.nltiles = 0; out(lone_folds(m, 8, true));\n"
+    got = run(tmp_path, body)
+    for (n, lone, b, c), f, g in zip(cases, got[::2], got[1::2]):
+        large = n * b >= 30 * 2**20
+        assert g == int(large), (n, lone, b, c)
+        assert f == int(large or lone >= 0.65 or (c and b == 8)), (n, lone, b, c)
+    assert got[-2:] == [0, 0]
