@@ -429,10 +429,8 @@ DevMaps phase_maps(const DevMaps& m, const Phase& p);
 // The id ranges and error word of every bucket (both setup paths).
 void set_id_bounds(const ogs_handle_s* h, DevMaps& m, unsigned int* err);
 
-// Per-type launchers (ogs_kern_*.cu).  Return a cudaError_t value.  k = 1
-// interleaved fields take the pipelined kernel over the exact-degree tiles
-// plus the direct kernel over the general tiles; every other case runs the
-// direct kernel over all tiles.
+// Per-type launchers (ogs_kern_*.cu; which kernels: ogs_launch.cuh).  Return a
+// cudaError_t value.
 int launch_f32(const DevMaps& m, const FieldArgs& f, int mode, int op, Pattern pat, void* stream);
 int launch_f64(const DevMaps& m, const FieldArgs& f, int mode, int op, Pattern pat, void* stream);
 int launch_i32(const DevMaps& m, const FieldArgs& f, int mode, int op, Pattern pat, void* stream);

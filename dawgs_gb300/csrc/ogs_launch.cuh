@@ -1,12 +1,13 @@
 // ogs_launch.cuh -- per-type launch dispatch shared by ogs_kern_*.cu.
 //
-// Scatter runs in node order where the handle's rows are numbered by first
-// member (ogs_scatter.cuh).  Otherwise exact-degree rows of GatherScatter run
+// Scatter of few components runs in node order where the handle's rows are
+// numbered by first member (ogs_scatter.cuh).  Otherwise exact-degree rows of GatherScatter run
 // on the warp pipeline with cp.async-staged gathers (ogs_async.cuh), those of
 // Gather, and of Scatter over rows in another order, on the register pipeline
 // of ogs_warp.cuh (-DOGS_GATHER_REGISTERS=0: everything on the cp.async one; -DOGS_ASYNC=0:
 // everything on the register one).  Rows above degree 8 run as wide tiles
-// (ogs_wide.cuh), or on the direct CTA kernel (ogs_kernels.cuh).  Building
+// (ogs_wide.cuh), or on the direct CTA kernel (ogs_kernels.cuh), which also takes
+// every row of calls with more than 2^27 components (units_fit).  Building
 // with -DOGS_KERNEL=2 runs the direct CTA kernel for every row instead (for
 // comparisons).
 //

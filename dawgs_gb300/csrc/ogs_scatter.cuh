@@ -9,7 +9,7 @@
 // bytes for each of the nnz - R other members and half a byte a node instead
 // of 4 (nnz + R) bytes, and the field's stores fill whole sectors.  What bounds
 // it is bandwidth: 24^3 p=7 fp64 moves 38.6 MB of gathered values, 56.6 MB of
-// field and 11 MB of rows and words in 21.5 us (28.7 us through the column
+// field and 11 MB of rows and words in 20.9 us (28.3 us through the column
 // lists), p=15 875 MB in 152 us (257), 32x32x16 p=5 permuted fp32 k=3 13.3 us
 // (20.5).  k is a constant: with k from 5 up as a number given at the launch,
 // every word took eight runs and a division, 20^3 p=7 fp64 k=5 82.7 us and k=8

@@ -8,9 +8,9 @@
 // tile's k parts as in ogs_async.cuh.  Before, a CTA took up to 256 rows
 // through their CSR lists, a thread a row and one load after the other, all
 // components in turn.  GatherScatter fp64, vertices of degree 24, us a call
-// before and now: 64^3 cells of six p=1 tetrahedra 69.8 -> 58.5, 20x20x16 of
-// p=3 with k=3 27.8 -> 17.0, 24^3 of p=2 in 4 arrays 43.8 -> 32.4, 32x32x24 of
-// p=3 27.3 -> 26.2.  Slower forms: four lanes a row with the members passed by
+// before and now: 64^3 cells of six p=1 tetrahedra 72.0 -> 59.3, 20x20x16 of
+// p=3 with k=3 26.0 -> 15.1, 24^3 of p=2 in 4 arrays 43.0 -> 31.2, 32x32x24 of
+// p=3 25.5 -> 24.8.  Slower forms: four lanes a row with the members passed by
 // shuffles (an fp64 add costs a warp 16 cycles of its pipe whatever lanes take
 // part), and the tiles at the head of the launch of the exact-degree rows (28-34
 // us in the last case, and that kernel 3 % slower where there are none).
