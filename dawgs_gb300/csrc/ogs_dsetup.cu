@@ -875,6 +875,13 @@ ogs_status build_device_layout(ogs_handle_s* h, const int32_t* rsT, const int32_
 
 }  // namespace
 
+int launch_wide_ids(const DevMaps& m, void* stream) {
+  if (m.nwide == 0) return 0;
+  k_wide_ids<<<nblocks(static_cast<int64_t>(m.nwide) * 32), kT, 0, static_cast<cudaStream_t>(stream)>>>(
+      m.wide, m.nwide, m.g.startsT, m.g.colsT, m.g.startsN, m.g.colsN, const_cast<uint32_t*>(m.wide_ids));
+  return cudaGetLastError();
+}
+
 ogs_status build_device_maps(ogs_handle_s* h, int64_t N, int64_t* ids, int kind, int unique, bool layout) {
   TraceRange trace("ogs_setup: maps on the GPU");
   if (kind == OGS_HALO)

@@ -333,7 +333,7 @@ struct HostLayout {
   std::vector<Tile> ltiles;        // see DevMaps
   std::vector<uint8_t> lmask8, lmask4, lmask1;  // host path only
   std::vector<Tile> wide;          // see DevMaps
-  std::vector<uint32_t> wide_ids;  // host path only
+  int64_t wide_units = 0;          // 32 ids each
   std::vector<Phase> phases;
   int64_t g_n = 0, g_nnzT = 0;  // general-bucket rows and T entries
   // lowest and highest local node each warp tile / general tile touches
@@ -407,6 +407,8 @@ inline bool scatter_share(const ogs_handle_s* h) { return h->nnzT * 4 >= h->N * 
 // they take.  None where rows of very different degree are neighbours and the
 // padding would outweigh the rows.
 int64_t wide_layout(const int32_t* starts, int64_t rows, std::vector<Tile>& wide);
+// Fills m.wide_ids from the general rows on `stream` (ogs_dsetup.cu); a cudaError_t value.
+int launch_wide_ids(const DevMaps& m, void* stream);
 // Whether a handle gets lone tiles for its n1 rows of degree 1 (the rows being
 // numbered by first member): from 55 % of its nodes on; which calls run over them
 // is up to lone_folds and lone_gathers.  Us a call without and with them, boxes of
