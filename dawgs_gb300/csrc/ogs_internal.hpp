@@ -286,18 +286,20 @@ inline bool lone_gathers(const DevMaps& m, int bytes) {
 
 // Whether a Scatter runs in node order (ogs_scatter.cuh): where the handle has
 // node words (rows numbered by first member) and most of its nodes take part
-// (scatter_share), for up to kScatterMaxK components.
-// A warp takes every component of a word, so more of them leave a small mesh
-// with few warps that each go through many rounds (eight runs a round: 1,000
+// (scatter_share), for components of up to kScatterNodeBytes a node: 8 of 8 bytes,
+// 16 of 4.  A warp takes every component of a word, so more of them leave a small
+// mesh with few warps that each go through many rounds (eight runs a round: 1,000
 // nodes k=1000 117 us against 3.9 through the column lists, 64 nodes k=20000
-// 2,459 against 7.9, 20^3 p=7 k=64 fp64 93 against 78, k=16 27.6 against 23.0).
-// Up to eight it is the faster one on boxes from 6^3 p=3 to 24^3 p=7, permuted
-// or not, fp32 and fp64 (0.55 to 1.0 of the time) but for fp64 k=4 and fp32 k=5
-// at 24^3 p=7 (74.1 and 61.2 us against 70.5 and 58.2).  Operators over caller
-// maps and the slices of host-buffer calls keep the tile kernels.
-constexpr int kScatterMaxK = 8;
-inline bool scatter_applies(const DevMaps& m, const FieldArgs& f, const Pattern& pat) {
-  return m.nodes.scatter && f.K <= kScatterMaxK && !f.is_many && !pat.gslib && pat.scatter_n <= 1;
+// 2,459 against 7.9, 20^3 p=7 k=64 fp64 93 against 78).  Through the column lists
+// / in node order, us: fp64 k=8 10^3 p=7 8.5 / 7.4, 24^3 p=7 134.8 / 130.1, 40^3
+// p=3 permuted 80.5 / 82.5, k=5 24^3 p=7 101.4 / 86.2; fp32 k=8 20^3 p=7 56.2 /
+// 43.9, k=14 10^3 p=7 11.0 / 8.5 and 20^3 p=7 87.4 / 86.8, k=16 12.1 / 9.5, 105.8 /
+// 114.0 and 40^3 p=3 permuted 109.1 / 120.9.  Operators over caller maps and the
+// slices of host-buffer calls keep the tile kernels.
+constexpr int kScatterNodeBytes = 64;
+OGS_HD constexpr int scatter_max_k(int bytes) { return kScatterNodeBytes / bytes; }
+inline bool scatter_applies(const DevMaps& m, const FieldArgs& f, const Pattern& pat, int bytes) {
+  return m.nodes.scatter && f.K <= scatter_max_k(bytes) && !f.is_many && !pat.gslib && pat.scatter_n <= 1;
 }
 
 // A slice of the warp and general tiles for the host-buffer pipeline: its

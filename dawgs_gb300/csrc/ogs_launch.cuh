@@ -62,7 +62,7 @@ inline int launch_typed(const DevMaps& m, const FieldArgs& f, int mode, int op, 
   cudaError_t e;
   if (mode == kModeGS) e = launch_op<T, kModeGS>(m, f, op, pat, s);
   else if (mode == kModeGather) e = launch_op<T, kModeGather>(m, f, op, pat, s);
-  else if (OGS_KERNEL == 0 && scatter_applies(m, f, pat)) e = launch_scatter<T>(m, f, pat, s);
+  else if (OGS_KERNEL == 0 && scatter_applies(m, f, pat, sizeof(T))) e = launch_scatter<T>(m, f, pat, s);
   else e = launch_mode<T, OGS_ADD, kModeScatter>(m, f, pat, s);  // a copy: op unused
   return static_cast<int>(e);
 }

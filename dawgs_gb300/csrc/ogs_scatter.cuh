@@ -103,23 +103,19 @@ inline cudaError_t launch_scatter_as(const DevMaps& m, const FieldArgs& f, cudaS
   return launch_scatter_block<T, K, NONLY, kScatterBlock>(m, f, s);
 }
 
-template <typename T, bool NONLY>
+// The instantiation of f.K components, from K down.
+template <typename T, bool NONLY, int K>
 inline cudaError_t launch_scatter_k(const DevMaps& m, const FieldArgs& f, cudaStream_t s) {
-  switch (f.K) {
-    case 1: return launch_scatter_as<T, 1, NONLY>(m, f, s);
-    case 2: return launch_scatter_as<T, 2, NONLY>(m, f, s);
-    case 3: return launch_scatter_as<T, 3, NONLY>(m, f, s);
-    case 4: return launch_scatter_as<T, 4, NONLY>(m, f, s);
-    case 5: return launch_scatter_as<T, 5, NONLY>(m, f, s);
-    case 6: return launch_scatter_as<T, 6, NONLY>(m, f, s);
-    case 7: return launch_scatter_as<T, 7, NONLY>(m, f, s);
-    default: return launch_scatter_as<T, 8, NONLY>(m, f, s);
+  if constexpr (K > 1) {
+    if (f.K < K) return launch_scatter_k<T, NONLY, K - 1>(m, f, s);
   }
+  return launch_scatter_as<T, K, NONLY>(m, f, s);
 }
 
 template <typename T>
 inline cudaError_t launch_scatter(const DevMaps& m, const FieldArgs& f, const Pattern& pat, cudaStream_t s) {
-  return pat.scatter_n ? launch_scatter_k<T, true>(m, f, s) : launch_scatter_k<T, false>(m, f, s);
+  constexpr int K = scatter_max_k(sizeof(T));
+  return pat.scatter_n ? launch_scatter_k<T, true, K>(m, f, s) : launch_scatter_k<T, false, K>(m, f, s);
 }
 
 }  // namespace ogsgb

@@ -31,6 +31,15 @@ def test_at_the_larger_ctas(cuda, oracle_mod, k, words, more):
         scattered(oracle_mod, random_ids(n, n // 3, seed=n, zero_frac=0.1), k, dtype)
 
 
+@pytest.mark.parametrize("k", [7, 8, 9, 13, 15, 16, 17])
+@pytest.mark.parametrize("n", [33, 4097, 140001])
+def test_components_up_to_the_tiles(cuda, oracle_mod, n, k):
+    """Each count of components is a kernel of its own up to 64 bytes a node."""
+    ids = random_ids(n, n // 3, seed=n + k, zero_frac=0.05)
+    for dtype in (np.float32, np.int32, np.float64, np.int64):
+        scattered(oracle_mod, ids, k, dtype)
+
+
 @pytest.mark.parametrize("k", [1, 3, 9])
 @pytest.mark.parametrize("zeros", [0.22, 0.28, 0.99])
 def test_where_few_nodes_take_part(cuda, oracle_mod, zeros, k):

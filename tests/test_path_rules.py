@@ -30,9 +30,10 @@ def test_scatter_in_node_order_takes_few_components(tmp_path):
     """A warp walks every component of its nodes, so large k goes to the tiles;
     no accepted k brings a component's place in a word near 32 bits."""
     body = "DevMaps m{}; m.nodes.nwords = 40; m.nodes.scatter = 1; FieldArgs f{}; Pattern p{0, 0, 0};\n"
-    body += "".join(f"f.K = {k}; out(scatter_applies(m, f, p));\n" for k in KS)
+    ks = KS + [16, 17]
+    body += "".join(f"f.K = {k}; out(scatter_applies(m, f, p, 8)); out(scatter_applies(m, f, p, 4));\n" for k in ks)
     got = run(tmp_path, body)
-    assert got == [1, 1, 1] + [0] * 8
+    assert got[::2] == [int(k <= 8) for k in ks] and got[1::2] == [int(k <= 16) for k in ks]
 
 
 def test_scatter_in_node_order_takes_handles_with_most_nodes_in_rows(tmp_path):
